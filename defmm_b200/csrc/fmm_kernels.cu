@@ -2160,14 +2160,7 @@ __global__ void k_scatter_rhs(const double2* __restrict__ pnear, const double2* 
   out[r * stride + perm[i]] = a;
 }
 
-// tp steps of a symmetric block: lane ls owns one source (y, qj) and meets
-// target (ls + step) mod tp; the target's running sum moves one lane down per
-// step.  TP = 32 fixes the segment width at compile time.
-// Target records in shared memory as two 16-byte arrays, (x, y) and (z, w)
-// with w the FP32 charge's bits (mixed path) or unused (FP64 path, the charge
-// in tq): one conflict-free 16-byte load from each per step.  Entry j holds
-// target j mod tp (j < 64), so step st of lane ls reads entry ls + st without
-// wrapping arithmetic.
+// Target charges of the mixed path ride in the second word of (z, w).
 __device__ __forceinline__ float2 charge_bits(double w) {
   const long long b = __double_as_longlong(w);
   return make_float2(__int_as_float((int)(b & 0xffffffffLL)), __int_as_float((int)(b >> 32)));
@@ -2176,54 +2169,81 @@ __device__ __forceinline__ double charge_word(float2 q) {
   return __longlong_as_double(((long long)(unsigned)__float_as_int(q.y) << 32) | (unsigned)__float_as_int(q.x));
 }
 
-template <bool MIXED, int TP>
-__device__ __forceinline__ void sym_steps(int ls, int tp_rt, double yx, double yy, double yz,
-                                          typename std::conditional<MIXED, float2, double2>::type qj,
-                                          const double2* trxy, const double2* trzw, const double2* tq,
-                                          double kappa,
-                                          typename std::conditional<MIXED, float2, double2>::type& accD,
-                                          typename std::conditional<MIXED, float2, double2>::type& accT) {
-  const int tp = TP ? TP : tp_rt;
-  const double2* txy = trxy + ls;
-  const double2* tzw = trzw + ls;
-  const double2* tql = tq + ls;
-#pragma unroll 8
-  for (int st = 0; st < tp; st++) {
-    const double2 a = txy[st], b = tzw[st];
-    if constexpr (MIXED) {
-      const float2 g = green32(a.x - yx, a.y - yy, b.x - yz, kappa);
-      const float2 qi = charge_bits(b.y);
-      accD.x = fmaf(g.x, qj.x, fmaf(-g.y, qj.y, accD.x));
-      accD.y = fmaf(g.x, qj.y, fmaf(g.y, qj.x, accD.y));
-      accT.x = fmaf(g.x, qi.x, fmaf(-g.y, qi.y, accT.x));
-      accT.y = fmaf(g.x, qi.y, fmaf(g.y, qi.x, accT.y));
-    } else {
-      const double2 g = green64(a.x - yx, a.y - yy, b.x - yz, kappa);
-      const double2 qi = tql[st];
-      accD.x = fma(g.x, qj.x, fma(-g.y, qj.y, accD.x));
-      accD.y = fma(g.x, qj.y, fma(g.y, qj.x, accD.y));
-      accT.x = fma(g.x, qi.x, fma(-g.y, qi.y, accT.x));
-      accT.y = fma(g.x, qi.y, fma(g.y, qi.x, accT.y));
-    }
-    accD.x = __shfl_sync(0xffffffffu, accD.x, ls + 1, tp);
-    accD.y = __shfl_sync(0xffffffffu, accD.y, ls + 1, tp);
-  }
+// exp(i k r) / r of one pair in FP64 (0 for R < 1e-16, P2P.hpp:66), without
+// the factor 1 / (4 pi), with kq = 2 k / pi.  An FP64 instruction takes two
+// issue cycles, every other one, so both counts matter (41 FP64 instructions
+// here, 48 and two conversions in green64): 1/r from the approximate
+// reciprocal square root by one cubic step y + y e (1/2 + 3/8 e),
+// e = 1 - R y^2 (|e| < 2^-19: the next term is below 2^-58); the phase in
+// quarter turns, r kq = n + u with |u| <= 1/2, u by one exactly rounded FMA
+// and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
+// (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
+// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20); R kept
+// away from zero by an integer maximum on its high word.
+__device__ __forceinline__ double2 green64_unscaled(double dx, double dy, double dz, double kq) {
+  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const bool skip = __double_as_longlong(R0) < 0x3C9CD2B297D889BCLL;  // R0 < 1e-16
+  const double R = __hiloint2double(max(__double2hiint(R0), 0x3C9CD2B2), __double2loint(R0));
+  const double y0 = rsqrt_approx64(R);
+  const double e = fma(-(R * y0), y0, 1.0);
+  const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+  const double r = R * y;
+  const double t = fma(r, kq, 6755399441055744.0);  // + 1.5 * 2^52
+  const double u = fma(r, kq, -(t - 6755399441055744.0));
+  const int q = __double2loint(t);
+  const double z = u * u;
+  double ps = fma(z, 5.633721016484235e-08, -3.598641754487236e-06);
+  ps = fma(z, ps, 0.00016044115029166428);
+  ps = fma(z, ps, -0.00468175413228242);
+  ps = fma(z, ps, 0.07969262624603957);
+  ps = fma(z, ps, -0.6459640975062443);
+  ps = fma(z, ps, 1.5707963267948966);
+  double pc = fma(z, -6.321892625650177e-09, 4.7106156592722383e-07);
+  pc = fma(z, pc, -2.5202036991591028e-05);
+  pc = fma(z, pc, 0.0009192602742250428);
+  pc = fma(z, pc, -0.020863480763315442);
+  pc = fma(z, pc, 0.2536695079010469);
+  pc = fma(z, pc, -1.2337005501361697);
+  pc = fma(z, pc, 1.0);
+  const double K = skip ? 0. : y;
+  const double sr = u * K * ps, cr = K * pc;
+  const double ss = (q & 1) ? cr : sr, cc = (q & 1) ? sr : cr;
+  // signs: sin negative in quadrants 2, 3; cos in 1, 2
+  return make_double2(__hiloint2double(__double2hiint(cc) ^ (int)((unsigned)(q + 1) << 30 & 0x80000000u),
+                                       __double2loint(cc)),
+                      __hiloint2double(__double2hiint(ss) ^ (int)((unsigned)q << 30 & 0x80000000u),
+                                       __double2loint(ss)));
 }
 
 // Symmetric blocks of the near field (Plan::sym_*): one CTA (4 warps) per
 // work item (part of the sources of one chunk of <= 32 targets), items taken
-// from a queue in the host's order of decreasing work.  A warp splits into segments
-// of tp = nextpow2(nt) lanes; lane l of a segment owns source l of the
-// segment's tp-source sub-tile and, over tp steps, meets every target
-// i = (l + step) mod tp.  One evaluation of G feeds both
-//   the target's partial  (an accumulator that moves one lane down per step
-//                          and ends in lane i), and
-//   the source's partial  (lane-local),
+// from a queue in the host's order of decreasing work.  A lane owns S
+// sources and meets the chunk's targets in blocks of 4, read from shared
+// memory by broadcast.  One evaluation of G feeds both
+//   the target's partial: 4 sums per block, over the lane's S sources; two
+//     exchange steps leave one target per lane (summed over 4 lanes), added
+//     to the lane's sum for this block in shared memory, and
+//   the source's partial (lane-local over all targets),
 // so each mirrored pair of interactions costs one kernel evaluation.  Target
 // partials of the item go to tpart (added per chunk by k_p2p_items); source
 // partials go to scratch and are added per source leaf by k_p2p_reduce.
+//
+// The sources of an item (thousands) fill the lanes whatever the number of
+// targets, which is only padded to a multiple of 4: 92-95% of the evaluated
+// pairs count, where segments of nextpow2(targets) lanes that passed the
+// targets' sums around gave 76-86%; and 8 independent evaluations per lane
+// keep the FP64 pipe fed (65% of its cycles on a 31k-point sphere).  The near
+// field of a 250k-point sphere in FP64 took 20.1 ms with the segments and
+// takes 15 ms so; of a 600k-point sphere in mixed precision 22.5 and 20 ms.
 template <bool MIXED>
-__global__ void __launch_bounds__(128) k_p2p_sym(DevPlan P, int64_t nwork, const int32_t* __restrict__ order,
+struct P2PSym {
+  static constexpr int S = 2;       // sources per lane
+  static constexpr int NB = 8;      // blocks of 4 targets in a chunk
+  typedef typename std::conditional<MIXED, float4, double2>::type A;  // (sum, compensation) or sum
+};
+
+template <bool MIXED>
+__global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, const int32_t* __restrict__ order,
                                                  const int32_t* __restrict__ item_chunk,
                                                  const int32_t* __restrict__ tfirst, const int32_t* __restrict__ tn,
                                                  const int64_t* __restrict__ ptr, const int32_t* __restrict__ sfirst,
@@ -2231,16 +2251,21 @@ __global__ void __launch_bounds__(128) k_p2p_sym(DevPlan P, int64_t nwork, const
                                                  const void* __restrict__ qv, double2* __restrict__ tpart,
                                                  void* __restrict__ scratch, unsigned long long* __restrict__ queue) {
   typedef typename std::conditional<MIXED, float2, double2>::type Q;
-  constexpr int RMAX = 128;
+  typedef P2PSym<MIXED> G;
+  typedef typename G::A Acc;
+  constexpr int RMAX = 128, S = G::S, NB = G::NB;
   const Q* q = static_cast<const Q*>(qv);
   Q* scr = static_cast<Q*>(scratch);
-  __shared__ double2 trxy[64], trzw[64];
-  __shared__ double2 tq[64];  // FP64 path: target charges
+  __shared__ double2 trxy[4 * NB], trzw[4 * NB];
+  __shared__ double2 tq[MIXED ? 1 : 4 * NB];  // FP64 path: target charges
+  __shared__ Acc tacc[4][NB][32];
   __shared__ int32_t rpre[RMAX + 1], rfst[RMAX];
   __shared__ int64_t roff[RMAX];
   __shared__ double2 red[4][32];
   __shared__ int64_t cur;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double kq = P.kappa * 0.63661977236758134308;  // 2 k / pi
+  const double scale = MIXED ? 1. : 1. / (4. * 3.14159265358979323846);
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
@@ -2250,30 +2275,25 @@ __global__ void __launch_bounds__(128) k_p2p_sym(DevPlan P, int64_t nwork, const
     const int64_t it = order[k];
     const int64_t ch = item_chunk[it];
     const int f = tfirst[ch], nt = tn[ch];
-    int tp = 4;
-    while (tp < nt) tp <<= 1;
-    const int ls = lane & (tp - 1);
-    if (threadIdx.x < 64) {
-      const int j = threadIdx.x, t = j & (tp - 1);
+    const int nb = (nt + 3) >> 2;
+    if (threadIdx.x < 4 * NB) {
+      const int t = threadIdx.x;
+      double2 xy = make_double2(0., 0.), zw = make_double2(0., 0.);
+      Q qt = Q{0, 0};
       if (t < nt) {
         const double* x = P.T_pos + 3 * (int64_t)(f + t);
-        const Q qt = q[f + t];
-        double w = 0.;
-        if constexpr (MIXED) {
-          w = charge_word(qt);
-        } else {
-          tq[j] = qt;
-        }
-        trxy[j] = make_double2(x[0], x[1]);
-        trzw[j] = make_double2(x[2], w);
-      } else {
-        trxy[j] = make_double2(0., 0.);
-        trzw[j] = make_double2(0., 0.);
-        tq[j] = make_double2(0., 0.);
+        qt = q[f + t];
+        xy = make_double2(x[0], x[1]);
+        zw.x = x[2];
       }
+      if constexpr (MIXED)
+        zw.y = charge_word(qt);
+      else
+        tq[t] = qt;
+      trxy[t] = xy;
+      trzw[t] = zw;
     }
-    float sr = 0.f, cr = 0.f, si = 0.f, ci = 0.f;  // mixed: compensated target sums
-    double pr = 0., pim = 0.;                      // FP64 target sums
+    for (int b = 0; b < nb; b++) tacc[warp][b][lane] = Acc{};
     const int64_t rb = ptr[it], re = ptr[it + 1];
     for (int64_t r0 = rb; r0 < re; r0 += RMAX) {
       const int nr = (int)min((int64_t)RMAX, re - r0);
@@ -2299,53 +2319,106 @@ __global__ void __launch_bounds__(128) k_p2p_sym(DevPlan P, int64_t nwork, const
       }
       __syncthreads();
       const int ntot = rpre[nr];
-      for (int base = warp * 32; base < ntot; base += 4 * 32) {
-        const int jj = base + lane;
-        const bool vj = jj < ntot;
-        double yx = 0., yy = 0., yz = 0.;
-        Q qj = Q{0, 0};
-        int64_t sidx = 0;
-        if (vj) {
-          int lo = 0, hi = nr - 1;  // last range with rpre <= jj
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (rpre[mid] <= jj) lo = mid; else hi = mid - 1;
+      for (int base = warp * 32 * S; base < ntot; base += 4 * 32 * S) {
+        double yx[S], yy[S], yz[S];
+        Q qj[S], accT[S];
+        int64_t sidx[S];
+#pragma unroll
+        for (int v = 0; v < S; v++) {
+          const int jj = base + 32 * v + lane;
+          yx[v] = yy[v] = yz[v] = 0.;
+          qj[v] = accT[v] = Q{0, 0};
+          sidx[v] = -1;
+          if (jj < ntot) {
+            int lo = 0, hi = nr - 1;  // last range with rpre <= jj
+            while (lo < hi) {
+              const int mid = (lo + hi + 1) >> 1;
+              if (rpre[mid] <= jj) lo = mid; else hi = mid - 1;
+            }
+            const int o = jj - rpre[lo];
+            const int64_t sj = (int64_t)rfst[lo] + o;
+            sidx[v] = roff[lo] + o;
+            const double* y = P.S_pos + 3 * sj;
+            yx[v] = y[0];
+            yy[v] = y[1];
+            yz[v] = y[2];
+            qj[v] = q[sj];
           }
-          const int o = jj - rpre[lo];
-          const int64_t sj = (int64_t)rfst[lo] + o;
-          sidx = roff[lo] + o;
-          const double* y = P.S_pos + 3 * sj;
-          yx = y[0];
-          yy = y[1];
-          yz = y[2];
-          qj = q[sj];
         }
-        Q accD = Q{0, 0}, accT = Q{0, 0};
         // no validity tests: padded targets and missing sources carry zero
-        // charges, and their target sums are never stored
-        if (tp == 32)
-          sym_steps<MIXED, 32>(ls, 32, yx, yy, yz, qj, trxy, trzw, tq, P.kappa, accD, accT);
-        else
-          sym_steps<MIXED, 0>(ls, tp, yx, yy, yz, qj, trxy, trzw, tq, P.kappa, accD, accT);
-        if constexpr (MIXED) {
-          kahan_add(sr, cr, accD.x);
-          kahan_add(si, ci, accD.y);
-        } else {
-          pr += accD.x;
-          pim += accD.y;
+        // charges, and their sums are never stored
+        for (int b = 0; b < nb; b++) {
+          Q d[4];
+#pragma unroll
+          for (int t = 0; t < 4; t++) {
+            const double2 a = trxy[4 * b + t], z = trzw[4 * b + t];
+            d[t] = Q{0, 0};
+#pragma unroll
+            for (int v = 0; v < S; v++) {
+              Q g, qi;
+              if constexpr (MIXED) {
+                g = green32(a.x - yx[v], a.y - yy[v], z.x - yz[v], P.kappa);
+                qi = charge_bits(z.y);
+              } else {
+                g = green64_unscaled(a.x - yx[v], a.y - yy[v], z.x - yz[v], kq);
+                qi = tq[4 * b + t];
+              }
+              d[t].x = fma(g.x, qj[v].x, fma(-g.y, qj[v].y, d[t].x));
+              d[t].y = fma(g.x, qj[v].y, fma(g.y, qj[v].x, d[t].y));
+              accT[v].x = fma(g.x, qi.x, fma(-g.y, qi.y, accT[v].x));
+              accT[v].y = fma(g.x, qi.y, fma(g.y, qi.x, accT[v].y));
+            }
+          }
+          // lanes with bit 4 keep targets 2, 3, the others 0, 1; then bit 3
+          // chooses the odd or the even one
+          const bool h1 = lane & 16, h0 = lane & 8;
+          Q k0 = h1 ? d[2] : d[0], k1 = h1 ? d[3] : d[1], s0 = h1 ? d[0] : d[2], s1 = h1 ? d[1] : d[3];
+          k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 16);
+          k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 16);
+          k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 16);
+          k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 16);
+          Q kk = h0 ? k1 : k0;
+          s0 = h0 ? k0 : k1;
+          kk.x += __shfl_xor_sync(0xffffffffu, s0.x, 8);
+          kk.y += __shfl_xor_sync(0xffffffffu, s0.y, 8);
+          Acc o = tacc[warp][b][lane];
+          if constexpr (MIXED) {
+            kahan_add(o.x, o.y, kk.x);
+            kahan_add(o.z, o.w, kk.y);
+          } else {
+            o.x += kk.x;
+            o.y += kk.y;
+          }
+          tacc[warp][b][lane] = o;
         }
-        if (vj) scr[sidx] = accT;
+#pragma unroll
+        for (int v = 0; v < S; v++)
+          if (sidx[v] >= 0) {
+            if constexpr (!MIXED) {
+              accT[v].x *= scale;
+              accT[v].y *= scale;
+            }
+            scr[sidx[v]] = accT[v];
+          }
       }
     }
-    if constexpr (MIXED) {
-      pr = (double)sr - (double)cr;
-      pim = (double)si - (double)ci;
+    for (int b = 0; b < nb; b++) {
+      const Acc o = tacc[warp][b][lane];
+      double pr, pim;
+      if constexpr (MIXED) {
+        pr = (double)o.x - (double)o.y;
+        pim = (double)o.z - (double)o.w;
+      } else {
+        pr = o.x * scale;
+        pim = o.y * scale;
+      }
+#pragma unroll
+      for (int w = 4; w; w >>= 1) {
+        pr += __shfl_xor_sync(0xffffffffu, pr, w);
+        pim += __shfl_xor_sync(0xffffffffu, pim, w);
+      }
+      if (!(lane & 7)) red[warp][4 * b + (lane >> 3 & 2) + (lane >> 3 & 1)] = make_double2(pr, pim);
     }
-    for (int o = tp; o < 32; o <<= 1) {  // segments of the warp hold the same targets
-      pr += __shfl_xor_sync(0xffffffffu, pr, o);
-      pim += __shfl_xor_sync(0xffffffffu, pim, o);
-    }
-    if (lane < tp) red[warp][lane] = make_double2(pr, pim);
     __syncthreads();
     if (threadIdx.x < nt) {
       double2 a = red[0][threadIdx.x];

@@ -437,3 +437,18 @@ def test_multifrequency_kernel_matches_direct_sums(gpu):
     assert rel(p[idx], ex) <= 1e-2  # the FMM's own error at order 5
     A.set_precision("mixed")
     assert rel(A.matvec(q), p) <= MIXED_TOL
+
+
+@pytest.mark.parametrize("ncrit", [5, 33, 61])
+def test_near_field_target_remainders(ncrit, gpu):
+    # leaves of every size up to ncrit: chunks of 1..32 targets (blocks of
+    # four with 0..3 padded ones), sources that do not fill the lanes, and
+    # coincident points in one leaf (their pairs are skipped, P2P.hpp:66)
+    p = W.sphere_surface(2500, seed=41, wavelengths=4).points
+    p[100] = p[7]
+    q = W.charges(len(p), 8)
+    A = make(p, p, 4, ncrit, 2 * np.pi * 2)
+    ref = A.matvec(q)
+    assert rel(ref, O.OracleFMM(p, p, 4, ncrit, 2 * np.pi * 2, -1).gemv(q)) <= FP64_TOL
+    A.set_precision("mixed")
+    assert rel(A.matvec(q), ref) <= MIXED_TOL

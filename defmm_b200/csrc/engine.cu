@@ -83,7 +83,8 @@ struct defmm_handle {
   const int32_t* d_p2p_order = nullptr;
   const int32_t *d_p2p_item_chunk = nullptr, *d_sym_item_chunk = nullptr;
   const int64_t *d_p2p_chunk_items = nullptr, *d_sym_chunk_items = nullptr;
-  double2* d_tpart = nullptr;  // near-field item partial sums (32 per item)
+  double2* d_tpart = nullptr;  // near-field item partial sums (32 per item and part)
+  int p2p_split = 1, sym_split = 1;  // parts per near-field item (near_split)
   unsigned long long* d_queue = nullptr;
   // symmetric near field (Plan::self_*, sym_*, red_*)
   const int64_t *d_self_ptr = nullptr, *d_sym_ptr = nullptr, *d_sym_soff = nullptr, *d_red_ptr = nullptr,
@@ -255,6 +256,21 @@ void free_plan_device(defmm_handle* h) {
   h->ops_prec = -1;
   h->dev_bytes = 0;
   h->has_out = false;
+}
+
+// Parts per near-field work item.  An item holds up to 8,192 sources of one
+// chunk, about half a millisecond on a full SM, and small problems have fewer
+// items than the chip has CTA slots (4 per SM).  Measured, whole and in
+// parts: the 287 items of the 5,003-point sphere 147 and 76 us, the 1,300 of
+// the 20,000-point cube 579 and 414 us, the 778 very uneven ones of blobs to
+// a sphere (three right-hand sides) 530 and 230 us.  Items are cut until
+// there are 8 per slot (16 cost the mixed 31k-point sphere 2%, 2 leave the
+// cube whole), but not below 512 sources on average (two rounds of a CTA).
+int near_split(int nsm, int64_t items, int64_t chunks, int64_t pairs, int64_t targets) {
+  if (items <= 0 || targets <= 0) return 1;
+  const int64_t want = (8 * 4 * (int64_t)nsm + items - 1) / items;
+  const double sources = (double)pairs / (double)targets * (double)chunks / (double)items;  // per item
+  return (int)std::max<int64_t>(1, std::min<int64_t>({want, (int64_t)(sources / 512.), 16}));
 }
 
 int upload_plan(defmm_handle* h) {
@@ -435,7 +451,14 @@ int upload_plan(defmm_handle* h) {
     h->plan_allocs.push_back(e);
     CK(cudaMemset(e, 0, sizeof(int)));
     d.err = static_cast<int*>(e);
-    const size_t nitem = (size_t)std::max<int64_t>(1, std::max(p.near_items(), p.near_sym_items()));
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t pairs = p.i_near;
+    h->p2p_split = near_split(h->nsm, p.near_items(), p.near_chunks(), pairs, (int64_t)p.T.perm.size());
+    h->sym_split = near_split(h->nsm, p.near_sym_items(), p.near_chunks(), pairs / 2, (int64_t)p.T.perm.size());
+    const size_t nitem = (size_t)std::max<int64_t>(
+        1, std::max(p.near_items() * h->p2p_split, p.near_sym_items() * h->sym_split));
     void* tp = nullptr;
     CK(cudaMalloc(&tp, nitem * 32 * sizeof(double2)));
     h->plan_allocs.push_back(tp);
@@ -445,9 +468,6 @@ int upload_plan(defmm_handle* h) {
     CK(cudaMalloc(&qc, 2 * sizeof(unsigned long long)));  // P2P (stream 2), M2L (main stream)
     h->plan_allocs.push_back(qc);
     h->d_queue = static_cast<unsigned long long*>(qc);
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev));
   }
   int64_t nS = (int64_t)p.S.perm.size(), nT = (int64_t)p.T.perm.size();
   if ((st = ensure(h, h->pnear, 16 * nT)) || (st = ensure(h, h->pfar, 16 * nT)) ||
@@ -695,7 +715,7 @@ int prepare_grouped(defmm_handle* h, int R) {
   g.lfT1 = p.sT.n;
   const int64_t nS = (int64_t)p.S.perm.size(), nT = (int64_t)p.T.perm.size();
   const size_t slot_b = (size_t)R * p.LL * cs;
-  const size_t nitem = (size_t)std::max<int64_t>(1, p.near_items());
+  const size_t nitem = (size_t)std::max<int64_t>(1, p.near_items() * h->p2p_split);
   int st;
   if ((st = ensure(h, g.q, (size_t)nS * R * cs)) || (st = ensure(h, g.pnear, (size_t)nT * R * 16)) ||
       (st = ensure(h, g.pfar, (size_t)nT * R * 16)) || (st = ensure(h, g.tpart, nitem * 32 * R * 16)) ||
@@ -800,21 +820,21 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
   if (h->use_sym) {  // own leaves, then symmetric blocks, then the mirrored partial sums
     dfb::launch_p2p(fp64, d, p.near_self_items(), h->d_self_order, nullptr, h->d_tfirst, h->d_tn,
                     h->d_self_ptr, h->d_self_sfirst, h->d_self_sn, h->q.p, (double2*)h->pnear.p, nullptr,
-                    h->d_queue, h->nsm, sn);
+                    1, h->d_queue, h->nsm, sn);
     dfb::launch_p2p_sym(fp64, d, p.near_sym_items(), h->d_sym_order, h->d_sym_item_chunk, h->d_tfirst,
                         h->d_tn, h->d_sym_ptr, h->d_sym_sfirst, h->d_sym_sn, h->d_sym_soff, h->q.p, h->d_tpart,
-                        h->pscr.p, h->d_queue, h->nsm, h->p2p_bps[fp64 ? 0 : 1], sn);
-    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_sym_chunk_items, h->d_tpart, (double2*)h->pnear.p,
-                          h->nsm, sn);
+                        h->pscr.p, h->sym_split, h->d_queue, h->nsm, h->p2p_bps[fp64 ? 0 : 1], sn);
+    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_sym_chunk_items, h->d_tpart, h->sym_split,
+                          (double2*)h->pnear.p, h->nsm, sn);
     dfb::launch_p2p_reduce(fp64, p.near_red_leaves(), h->d_red_first, h->d_red_n, h->d_red_ptr,
                            h->d_red_off, h->pscr.p, (double2*)h->pnear.p, h->nsm, sn);
     nl_ += (p.near_self_items() ? 1 : 0) + (p.near_sym_items() ? 2 : 0) + (p.near_red_leaves() ? 1 : 0);
   } else {  // every interaction from the target side, in items
     dfb::launch_p2p(fp64, d, p.near_items(), h->d_p2p_order, h->d_p2p_item_chunk, h->d_tfirst, h->d_tn,
-                    h->d_p2p_ptr, h->d_sfirst, h->d_sn, h->q.p, (double2*)h->pnear.p, h->d_tpart, h->d_queue,
-                    h->nsm, sn);
-    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, h->d_tpart, (double2*)h->pnear.p,
-                          h->nsm, sn);
+                    h->d_p2p_ptr, h->d_sfirst, h->d_sn, h->q.p, (double2*)h->pnear.p, h->d_tpart, h->p2p_split,
+                    h->d_queue, h->nsm, sn);
+    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, h->d_tpart, h->p2p_split,
+                          (double2*)h->pnear.p, h->nsm, sn);
     nl_ += p.near_items() ? 2 : 0;
   }
   if (h->events) cudaEventRecord(h->ev[2 * PH_P2P + 1], sn);
@@ -1021,10 +1041,10 @@ int run_gemv_grouped(defmm_handle* h, const double2* qin, int64_t stride_in, dou
     if (h->events) CK(cudaEventRecord(e0, sn));
     dfb::launch_p2p_rhs(fp64, d, p.near_items(), h->d_p2p_order, h->d_p2p_item_chunk, h->d_tfirst,
                         h->d_tn, h->d_p2p_ptr, h->d_sfirst, h->d_sn, g.q.p, R, (double2*)g.pnear.p,
-                        (double2*)g.tpart.p, h->d_queue, h->nsm, h->p2p_bps[pi], sn);
-    dfb::launch_p2p_items_rhs(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, (const double2*)g.tpart.p, R,
+                        (double2*)g.tpart.p, h->p2p_split, h->d_queue, h->nsm, h->p2p_bps[pi], sn);
+    dfb::launch_p2p_items_rhs(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, (const double2*)g.tpart.p, h->p2p_split, R,
                               (double2*)g.pnear.p, h->nsm, sn);
-    nk += p.near_items() ? (R + 7) / 8 + 1 : 0;
+    nk += p.near_items() ? R / 8 + (R % 8 + 3) / 4 + 1 : 0;
     if (h->events) {
       CK(cudaEventRecord(e1, sn));
       CK(cudaEventSynchronize(e1));

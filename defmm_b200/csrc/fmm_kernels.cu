@@ -1651,32 +1651,6 @@ __global__ void __launch_bounds__(128) k_l2p(DevPlan P, const int32_t* __restric
 // sin/cos of the reduced angle are evaluated in FP32 by their Taylor series
 // to degree 13/12, 1/(4 pi r) and the complex products in FP32; every
 // product is accumulated in FP64.
-__device__ __forceinline__ void sincos_reduced(double theta, float& s, float& c) {
-  // theta = n pi + x, |x| <= pi/2 (FP64 reduction; n pi exact inside the FMA)
-  const double n = rint(theta * 0.31830988618379067154);  // 1/pi
-  const float x = (float)fma(-n, 3.14159265358979323846, theta);
-  const float x2 = x * x;
-  // sin x = x (1 - x^2/3! + ... + x^12/13!), cos x = 1 - x^2/2! + ... + x^12/12!
-  // (Taylor; truncation < 7e-10 on [-pi/2, pi/2])
-  float ps = fmaf(x2, 1.6059043836821613e-10f, -2.5052108385441720e-08f);
-  ps = fmaf(x2, ps, 2.7557319223985893e-06f);
-  ps = fmaf(x2, ps, -1.9841269841269841e-04f);
-  ps = fmaf(x2, ps, 8.3333333333333333e-03f);
-  ps = fmaf(x2, ps, -1.6666666666666667e-01f);
-  ps = fmaf(x2, ps, 1.0f);
-  float pc = fmaf(x2, 2.0876756987868099e-09f, -2.7557319223985891e-07f);
-  pc = fmaf(x2, pc, 2.4801587301587302e-05f);
-  pc = fmaf(x2, pc, -1.3888888888888889e-03f);
-  pc = fmaf(x2, pc, 4.1666666666666667e-02f);
-  pc = fmaf(x2, pc, -0.5f);
-  pc = fmaf(x2, pc, 1.0f);
-  // (-1)^n on both
-  const float sg = (__double2int_rn(n) & 1) ? -1.0f : 1.0f;
-  s = sg * x * ps;
-  c = sg * pc;
-}
-
-
 // Near field, tiled: one CTA (4 warps) per work item (part of the sources of
 // one chunk of <= 32 target particles of one leaf); CTAs take items from a
 // global queue in the host's order of decreasing work.  The chunk's source ranges are streamed through shared
@@ -1685,7 +1659,7 @@ __device__ __forceinline__ void sincos_reduced(double theta, float& s, float& c)
 // groups take interleaved sources of the tile, two at a time.  Partial sums
 // are reduced in FP64 through shuffles and shared memory; each target is
 // written once.
-//   MIXED = false: FP64 throughout (P2P.hpp:43-79 arithmetic, p2p_pair64).
+//   MIXED = false: FP64 throughout (P2P.hpp:43-79, green64).
 //   MIXED = true : difference vector, r^2, 1/r and the reduction of k r in
 //   FP64; sin/cos of the reduced angle, 1/(4 pi r) and the complex products
 //   in FP32 with compensated sums (p2p_pair_mixed).
@@ -1701,26 +1675,51 @@ __device__ __forceinline__ double rsqrt_approx64(double x) {
   return y;
 }
 
-// One FP64 source/target interaction.
-__device__ __forceinline__ void p2p_pair64(double x0, double x1, double x2, double2 a, double2 b, double2 qd,
-                                           double kappa, double& pr, double& pim) {
-  const double pi4m1 = 1. / (4. * 3.14159265358979323846);
-  const double dx = x0 - a.x, dy = x1 - a.y, dz = x2 - b.x;
-  const double R = fma(dx, dx, fma(dy, dy, dz * dz));
-  if (R < 1.e-16) return;  // self / duplicate pairs (P2P.hpp:66)
-  // 1/sqrt(R): approximate FP64 estimate, two Newton steps (quadratic)
-  double y = rsqrt_approx64(R);
-  const double hR = 0.5 * R;
-  y = y * fma(-hR * y, y, 1.5);
-  y = y * fma(-hR * y, y, 1.5);
-  const double rr = y * R * kappa;
-  const double K = y * pi4m1;
-  double sn_, cs_;
-  sincos_cw(rr, sn_, cs_);
-  cs_ *= K;
-  sn_ *= K;
-  pr = fma(cs_, qd.x, fma(-sn_, qd.y, pr));
-  pim = fma(cs_, qd.y, fma(sn_, qd.x, pim));
+// exp(i k r) / r of one pair in FP64 (0 for R < 1e-16, P2P.hpp:66), without
+// the factor 1 / (4 pi), with kq = 2 k / pi.  An FP64 instruction takes two
+// issue cycles, every other one, so both counts matter (41 FP64 instructions
+// here; the reduction by pi/2 in two parts with rint and Taylor series took
+// 48 and two conversions): 1/r from the approximate
+// reciprocal square root by one cubic step y + y e (1/2 + 3/8 e),
+// e = 1 - R y^2 (|e| < 2^-19: the next term is below 2^-58); the phase in
+// quarter turns, r kq = n + u with |u| <= 1/2, u by one exactly rounded FMA
+// and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
+// (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
+// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20); R kept
+// away from zero by an integer maximum on its high word.
+__device__ __forceinline__ double2 green64(double dx, double dy, double dz, double kq) {
+  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const bool skip = __double_as_longlong(R0) < 0x3C9CD2B297D889BCLL;  // R0 < 1e-16
+  const double R = __hiloint2double(max(__double2hiint(R0), 0x3C9CD2B2), __double2loint(R0));
+  const double y0 = rsqrt_approx64(R);
+  const double e = fma(-(R * y0), y0, 1.0);
+  const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+  const double r = R * y;
+  const double t = fma(r, kq, 6755399441055744.0);  // + 1.5 * 2^52
+  const double u = fma(r, kq, -(t - 6755399441055744.0));
+  const int q = __double2loint(t);
+  const double z = u * u;
+  double ps = fma(z, 5.633721016484235e-08, -3.598641754487236e-06);
+  ps = fma(z, ps, 0.00016044115029166428);
+  ps = fma(z, ps, -0.00468175413228242);
+  ps = fma(z, ps, 0.07969262624603957);
+  ps = fma(z, ps, -0.6459640975062443);
+  ps = fma(z, ps, 1.5707963267948966);
+  double pc = fma(z, -6.321892625650177e-09, 4.7106156592722383e-07);
+  pc = fma(z, pc, -2.5202036991591028e-05);
+  pc = fma(z, pc, 0.0009192602742250428);
+  pc = fma(z, pc, -0.020863480763315442);
+  pc = fma(z, pc, 0.2536695079010469);
+  pc = fma(z, pc, -1.2337005501361697);
+  pc = fma(z, pc, 1.0);
+  const double K = skip ? 0. : y;
+  const double sr = u * K * ps, cr = K * pc;
+  const double ss = (q & 1) ? cr : sr, cc = (q & 1) ? sr : cr;
+  // signs: sin negative in quadrants 2, 3; cos in 1, 2
+  return make_double2(__hiloint2double(__double2hiint(cc) ^ (int)((unsigned)(q + 1) << 30 & 0x80000000u),
+                                       __double2loint(cc)),
+                      __hiloint2double(__double2hiint(ss) ^ (int)((unsigned)q << 30 & 0x80000000u),
+                                       __double2loint(ss)));
 }
 
 // Compensated (Kahan) FP32 summation: s - c carries the sum.
@@ -1737,7 +1736,8 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
 // FP32 for 1/(4 pi r).  k r = n pi + x with n read from the
 // low mantissa bits of k r / pi + 1.5 * 2^52 (exact for k r / pi < 2^51) and
 // x = k r - n pi in FP64; sin/cos of x by the FP32 Taylor polynomials of
-// sincos_reduced, (-1)^n applied to both.
+// degree 13 and 12 (truncation below 7e-10 on [-pi/2, pi/2]), (-1)^n applied
+// to both.
 __device__ __forceinline__ void p2p_pair_mixed(double x0, double x1, double x2, double2 a, double2 b, double kappa,
                                                float& sr, float& cr, float& si, float& ci) {
   const double dx = x0 - a.x, dy = x1 - a.y, dz = x2 - b.x;
@@ -1778,7 +1778,7 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
                                                    const int64_t* __restrict__ ptr, const int32_t* __restrict__ sfirst,
                                                    const int32_t* __restrict__ sn, const void* __restrict__ qv,
                                                    double2* __restrict__ pnear, double2* __restrict__ tpart,
-                                                   unsigned long long* __restrict__ queue) {
+                                                   int split, unsigned long long* __restrict__ queue) {
   constexpr int TS = 512;
   typedef typename std::conditional<MIXED, float2, double2>::type Q;
   const Q* q = static_cast<const Q*>(qv);
@@ -1787,13 +1787,15 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
   __shared__ double2 red[4][32];
   __shared__ int64_t cur;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double kq = P.kappa * 0.63661977236758134308;  // 2 k / pi
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
     __syncthreads();
     const int64_t k = cur;
-    if (k >= nitem) break;
-    const int64_t it = order[k];
+    if (k >= nitem * split) break;
+    const int64_t it = order[k / split];
+    int tile = split - (int)(k % split);  // tiles until this part's first one, counted from split
     const int64_t ch = item_chunk ? item_chunk[it] : it;
     const int f = tfirst[ch], nt = tn[ch];
     int tp = 1;
@@ -1810,11 +1812,12 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
     while (r < re) {
       // fill one tile from consecutive ranges (uniform control flow)
       int fill = 0;
-      __syncthreads();
+      const bool mine = tile++ % split == 0;
+      if (mine) __syncthreads();
       while (r < re && fill < TS) {
         const int s0 = sfirst[r], ns = sn[r];
         const int take = min(ns - off, TS - fill);
-        for (int t = threadIdx.x; t < take; t += blockDim.x) {
+        for (int t = mine ? threadIdx.x : take; t < take; t += blockDim.x) {
           const int64_t sj = (int64_t)s0 + off + t;
           const double* y = P.S_pos + 3 * sj;
           sa[fill + t] = make_double2(y[0], y[1]);
@@ -1835,6 +1838,7 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
           off = 0;
         }
       }
+      if (!mine) continue;
       __syncthreads();
       int j = gid;
       if constexpr (MIXED) {
@@ -1844,16 +1848,21 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
         }
         if (j < fill) p2p_pair_mixed(x0, x1, x2, sa[j], sb[j], P.kappa, sr, cr, si, ci);
       } else {
-        for (; j + G < fill; j += 2 * G) {
-          p2p_pair64(x0, x1, x2, sa[j], sb[j], sc[j], P.kappa, pr, pim);
-          p2p_pair64(x0, x1, x2, sa[j + G], sb[j + G], sc[j + G], P.kappa, pr, pim);
+#pragma unroll 4
+        for (; j < fill; j += G) {
+          const double2 a = sa[j], qd = sc[j];
+          const double2 g = green64(x0 - a.x, x1 - a.y, x2 - sb[j].x, kq);
+          pr = fma(g.x, qd.x, fma(-g.y, qd.y, pr));
+          pim = fma(g.x, qd.y, fma(g.y, qd.x, pim));
         }
-        if (j < fill) p2p_pair64(x0, x1, x2, sa[j], sb[j], sc[j], P.kappa, pr, pim);
       }
     }
     if constexpr (MIXED) {
       pr = (double)sr - (double)cr;
       pim = (double)si - (double)ci;
+    } else {
+      pr *= 1. / (4. * 3.14159265358979323846);
+      pim *= 1. / (4. * 3.14159265358979323846);
     }
     for (int o = tp; o < 32; o <<= 1) {
       pr += __shfl_xor_sync(0xffffffffu, pr, o);
@@ -1868,7 +1877,7 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
         a.y += red[w][threadIdx.x].y;
       }
       if (tpart)
-        tpart[it * 32 + threadIdx.x] = a;  // item partial, added per chunk by k_p2p_items
+        tpart[(it * split + k % split) * 32 + threadIdx.x] = a;  // item partial, added per chunk by k_p2p_items
       else
         pnear[f + threadIdx.x] = a;
     }
@@ -1878,13 +1887,13 @@ __global__ void __launch_bounds__(128) k_p2p_tiled(DevPlan P, int64_t nitem, con
 // Item partial sums of the near field into p, per chunk in item order.
 __global__ void k_p2p_items(int64_t nchunk, const int32_t* __restrict__ tfirst, const int32_t* __restrict__ tn,
                             const int64_t* __restrict__ chunk_items, const double2* __restrict__ tpart,
-                            double2* __restrict__ pnear) {
+                            int split, double2* __restrict__ pnear) {
   const int t = threadIdx.x & 31;
   for (int64_t ch = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ch < nchunk;
        ch += (int64_t)gridDim.x * (blockDim.x >> 5)) {
     if (t >= tn[ch]) continue;
     double ar = 0., ai = 0.;
-    for (int64_t it = chunk_items[ch]; it < chunk_items[ch + 1]; it++) {
+    for (int64_t it = chunk_items[ch] * split; it < chunk_items[ch + 1] * split; it++) {
       const double2 v = tpart[it * 32 + t];
       ar += v.x;
       ai += v.y;
@@ -1897,24 +1906,9 @@ __global__ void k_p2p_items(int64_t nchunk, const int32_t* __restrict__ tfirst, 
 }
 
 // ----------------------------------------------------- symmetric near field --
-// G(x, y) = exp(i k r) / (4 pi r) of one pair (0 for R < 1e-16, P2P.hpp:66),
-// with the arithmetic of p2p_pair<false> (FP64) or p2p_pair_mixed (FP32
-// after the FP64 r and k r reduction).
-// Branch-free: a pair with R < 1e-16 is evaluated at R = 1 and scaled by 0.
-__device__ __forceinline__ double2 green64(double dx, double dy, double dz, double kappa) {
-  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
-  const bool skip = R0 < 1.e-16;
-  const double R = skip ? 1. : R0;
-  const double pi4m1 = skip ? 0. : 1. / (4. * 3.14159265358979323846);
-  double y = rsqrt_approx64(R);
-  const double hR = 0.5 * R;
-  y = y * fma(-hR * y, y, 1.5);
-  y = y * fma(-hR * y, y, 1.5);
-  const double K = y * pi4m1;
-  double sn_, cs_;
-  sincos_cw(y * R * kappa, sn_, cs_);
-  return make_double2(cs_ * K, sn_ * K);
-}
+// G(x, y) = exp(i k r) / (4 pi r) of one pair (0 for R < 1e-16, P2P.hpp:66)
+// with the arithmetic of p2p_pair_mixed.  Branch-free: a pair with R < 1e-16
+// is evaluated at R = 1 and scaled by 0.
 __device__ __forceinline__ float2 green32(double dx, double dy, double dz, double kappa) {
   const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
   const bool skip = R0 < 1.e-16;
@@ -1968,7 +1962,7 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
                                                  const int64_t* __restrict__ ptr, const int32_t* __restrict__ sfirst,
                                                  const int32_t* __restrict__ sn, const void* __restrict__ qv, int R,
                                                  int r0, double2* __restrict__ pnear, double2* __restrict__ tpart,
-                                                 unsigned long long* __restrict__ queue) {
+                                                 int split, unsigned long long* __restrict__ queue) {
   typedef P2PRhsCfg<MIXED, RB> G;
   constexpr int TS = G::TS;
   typedef typename G::Q Q;
@@ -1980,13 +1974,15 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
   double2* red = reinterpret_cast<double2*>(sq + TS * RB);  // [4][32][RB]
   __shared__ int64_t cur;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double kq = P.kappa * 0.63661977236758134308;  // 2 k / pi
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
     __syncthreads();
     const int64_t k = cur;
-    if (k >= nitem) break;
-    const int64_t it = order[k];
+    if (k >= nitem * split) break;
+    const int64_t it = order[k / split];
+    int tile = split - (int)(k % split);  // as in k_p2p_tiled
     const int64_t ch = item_chunk ? item_chunk[it] : it;
     const int f = tfirst[ch], nt = tn[ch];
     int tp = 1;
@@ -2003,17 +1999,18 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
     int off = 0;
     while (r < re) {
       int fill = 0;
-      __syncthreads();
+      const bool mine = tile++ % split == 0;
+      if (mine) __syncthreads();
       while (r < re && fill < TS) {
         const int s0 = sfirst[r], ns = sn[r];
         const int take = min(ns - off, TS - fill);
-        for (int t = threadIdx.x; t < take; t += blockDim.x) {
+        for (int t = mine ? threadIdx.x : take; t < take; t += blockDim.x) {
           const int64_t sj = (int64_t)s0 + off + t;
           const double* y = P.S_pos + 3 * sj;
           sa[fill + t] = make_double2(y[0], y[1]);
           sb[fill + t] = make_double2(y[2], 0.);
         }
-        for (int t = threadIdx.x; t < take * RB; t += blockDim.x) {
+        for (int t = mine ? threadIdx.x : take * RB; t < take * RB; t += blockDim.x) {
           const int64_t sj = (int64_t)s0 + off + t / RB;
           sq[fill * RB + t] = q[sj * R + r0 + t % RB];
         }
@@ -2024,6 +2021,7 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
           off = 0;
         }
       }
+      if (!mine) continue;
       __syncthreads();
       if constexpr (MIXED) {
         // FP32 products summed in FP32 over at most kFlush sources of this
@@ -2069,7 +2067,7 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
         for (int j = gid; j < fill; j += GS) {
           const double2 a = sa[j], bz = sb[j];
           const Q* qj = sq + j * RB;
-          const double2 g = green64(x0 - a.x, x1 - a.y, x2 - bz.x, P.kappa);
+          const double2 g = green64(x0 - a.x, x1 - a.y, x2 - bz.x, kq);
 #pragma unroll
           for (int b = 0; b < RB; b++) {
             const double2 qq = qj[b];
@@ -2081,6 +2079,10 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
     }
 #pragma unroll
     for (int b = 0; b < RB; b++) {
+      if constexpr (!MIXED) {
+        acc[b].x *= 1. / (4. * 3.14159265358979323846);
+        acc[b].y *= 1. / (4. * 3.14159265358979323846);
+      }
       for (int o = tp; o < 32; o <<= 1) {
         acc[b].x += __shfl_xor_sync(0xffffffffu, acc[b].x, o);
         acc[b].y += __shfl_xor_sync(0xffffffffu, acc[b].y, o);
@@ -2096,7 +2098,7 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
         a.y += red[(w * 32 + t) * RB + b].y;
       }
       if (tpart)
-        tpart[(it * 32 + t) * R + r0 + b] = a;
+        tpart[((it * split + k % split) * 32 + t) * R + r0 + b] = a;
       else
         pnear[(int64_t)(f + t) * R + r0 + b] = a;
     }
@@ -2106,7 +2108,7 @@ __global__ void __launch_bounds__(128) k_p2p_rhs(DevPlan P, int64_t nitem, const
 // Item partial sums of the near field into p for R right-hand sides, per
 // chunk in item order (k_p2p_items with R sums per target).
 __global__ void k_p2p_items_rhs(int64_t nchunk, const int32_t* __restrict__ tfirst, const int32_t* __restrict__ tn,
-                                const int64_t* __restrict__ chunk_items, const double2* __restrict__ tpart, int R,
+                                const int64_t* __restrict__ chunk_items, const double2* __restrict__ tpart, int split, int R,
                                 double2* __restrict__ pnear) {
   const int64_t per = 32 * (int64_t)R;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nchunk * per;
@@ -2115,7 +2117,7 @@ __global__ void k_p2p_items_rhs(int64_t nchunk, const int32_t* __restrict__ tfir
     const int t = (int)((w % per) / R), rr = (int)(w % R);
     if (t >= tn[ch]) continue;
     double ar = 0., ai = 0.;
-    for (int64_t it = chunk_items[ch]; it < chunk_items[ch + 1]; it++) {
+    for (int64_t it = chunk_items[ch] * split; it < chunk_items[ch + 1] * split; it++) {
       const double2 v = tpart[(it * 32 + t) * R + rr];
       ar += v.x;
       ai += v.y;
@@ -2169,55 +2171,10 @@ __device__ __forceinline__ double charge_word(float2 q) {
   return __longlong_as_double(((long long)(unsigned)__float_as_int(q.y) << 32) | (unsigned)__float_as_int(q.x));
 }
 
-// exp(i k r) / r of one pair in FP64 (0 for R < 1e-16, P2P.hpp:66), without
-// the factor 1 / (4 pi), with kq = 2 k / pi.  An FP64 instruction takes two
-// issue cycles, every other one, so both counts matter (41 FP64 instructions
-// here, 48 and two conversions in green64): 1/r from the approximate
-// reciprocal square root by one cubic step y + y e (1/2 + 3/8 e),
-// e = 1 - R y^2 (|e| < 2^-19: the next term is below 2^-58); the phase in
-// quarter turns, r kq = n + u with |u| <= 1/2, u by one exactly rounded FMA
-// and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
-// (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
-// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20); R kept
-// away from zero by an integer maximum on its high word.
-__device__ __forceinline__ double2 green64_unscaled(double dx, double dy, double dz, double kq) {
-  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
-  const bool skip = __double_as_longlong(R0) < 0x3C9CD2B297D889BCLL;  // R0 < 1e-16
-  const double R = __hiloint2double(max(__double2hiint(R0), 0x3C9CD2B2), __double2loint(R0));
-  const double y0 = rsqrt_approx64(R);
-  const double e = fma(-(R * y0), y0, 1.0);
-  const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
-  const double r = R * y;
-  const double t = fma(r, kq, 6755399441055744.0);  // + 1.5 * 2^52
-  const double u = fma(r, kq, -(t - 6755399441055744.0));
-  const int q = __double2loint(t);
-  const double z = u * u;
-  double ps = fma(z, 5.633721016484235e-08, -3.598641754487236e-06);
-  ps = fma(z, ps, 0.00016044115029166428);
-  ps = fma(z, ps, -0.00468175413228242);
-  ps = fma(z, ps, 0.07969262624603957);
-  ps = fma(z, ps, -0.6459640975062443);
-  ps = fma(z, ps, 1.5707963267948966);
-  double pc = fma(z, -6.321892625650177e-09, 4.7106156592722383e-07);
-  pc = fma(z, pc, -2.5202036991591028e-05);
-  pc = fma(z, pc, 0.0009192602742250428);
-  pc = fma(z, pc, -0.020863480763315442);
-  pc = fma(z, pc, 0.2536695079010469);
-  pc = fma(z, pc, -1.2337005501361697);
-  pc = fma(z, pc, 1.0);
-  const double K = skip ? 0. : y;
-  const double sr = u * K * ps, cr = K * pc;
-  const double ss = (q & 1) ? cr : sr, cc = (q & 1) ? sr : cr;
-  // signs: sin negative in quadrants 2, 3; cos in 1, 2
-  return make_double2(__hiloint2double(__double2hiint(cc) ^ (int)((unsigned)(q + 1) << 30 & 0x80000000u),
-                                       __double2loint(cc)),
-                      __hiloint2double(__double2hiint(ss) ^ (int)((unsigned)q << 30 & 0x80000000u),
-                                       __double2loint(ss)));
-}
-
 // Symmetric blocks of the near field (Plan::sym_*): one CTA (4 warps) per
-// work item (part of the sources of one chunk of <= 32 targets), items taken
-// from a queue in the host's order of decreasing work.  A lane owns S
+// work item, or part of one (part of the sources of one chunk of <= 32
+// targets), taken from a queue in the host's order of decreasing work; part p
+// of split takes every split-th round of 256 sources.  A lane owns S
 // sources and meets the chunk's targets in blocks of 4, read from shared
 // memory by broadcast.  One evaluation of G feeds both
 //   the target's partial: 4 sums per block, over the lane's S sources; two
@@ -2249,7 +2206,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
                                                  const int64_t* __restrict__ ptr, const int32_t* __restrict__ sfirst,
                                                  const int32_t* __restrict__ sn, const int64_t* __restrict__ soff,
                                                  const void* __restrict__ qv, double2* __restrict__ tpart,
-                                                 void* __restrict__ scratch, unsigned long long* __restrict__ queue) {
+                                                 void* __restrict__ scratch, int split, unsigned long long* __restrict__ queue) {
   typedef typename std::conditional<MIXED, float2, double2>::type Q;
   typedef P2PSym<MIXED> G;
   typedef typename G::A Acc;
@@ -2271,8 +2228,9 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
     if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
     __syncthreads();
     const int64_t k = cur;
-    if (k >= nwork) break;
-    const int64_t it = order[k];
+    if (k >= nwork * split) break;
+    const int64_t it = order[k / split];
+    const int part = (int)(k % split);
     const int64_t ch = item_chunk[it];
     const int f = tfirst[ch], nt = tn[ch];
     const int nb = (nt + 3) >> 2;
@@ -2319,7 +2277,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
       }
       __syncthreads();
       const int ntot = rpre[nr];
-      for (int base = warp * 32 * S; base < ntot; base += 4 * 32 * S) {
+      for (int base = (part * 4 + warp) * 32 * S; base < ntot; base += split * 4 * 32 * S) {
         double yx[S], yy[S], yz[S];
         Q qj[S], accT[S];
         int64_t sidx[S];
@@ -2360,7 +2318,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
                 g = green32(a.x - yx[v], a.y - yy[v], z.x - yz[v], P.kappa);
                 qi = charge_bits(z.y);
               } else {
-                g = green64_unscaled(a.x - yx[v], a.y - yy[v], z.x - yz[v], kq);
+                g = green64(a.x - yx[v], a.y - yy[v], z.x - yz[v], kq);
                 qi = tq[4 * b + t];
               }
               d[t].x = fma(g.x, qj[v].x, fma(-g.y, qj[v].y, d[t].x));
@@ -2426,7 +2384,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
         a.x += red[w][threadIdx.x].x;
         a.y += red[w][threadIdx.x].y;
       }
-      tpart[it * 32 + threadIdx.x] = a;
+      tpart[(it * split + part) * 32 + threadIdx.x] = a;
     }
   }
 }
@@ -2797,38 +2755,39 @@ void launch_scatter(const double2* pnear, const double2* pfar, const int32_t* pe
 
 void launch_p2p(bool fp64, const DevPlan& dp, int64_t nitem, const int32_t* order, const int32_t* item_chunk,
                 const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst, const int32_t* sn,
-                const void* q, double2* pnear, double2* tpart, unsigned long long* queue, int nsm, cudaStream_t s) {
+                const void* q, double2* pnear, double2* tpart, int split, unsigned long long* queue, int nsm,
+                cudaStream_t s) {
   if (!nitem) return;
   cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
-  const int grid = (int)std::min<int64_t>(nitem, (int64_t)nsm * 16);
+  const int grid = (int)std::min<int64_t>(nitem * split, (int64_t)nsm * 16);
   if (fp64)
     k_p2p_tiled<false><<<grid, 128, 0, s>>>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, pnear,
-                                            tpart, queue);
+                                            tpart, split, queue);
   else
     k_p2p_tiled<true><<<grid, 128, 0, s>>>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, pnear,
-                                           tpart, queue);
+                                           tpart, split, queue);
 }
 
 void launch_p2p_items(int64_t nchunk, const int32_t* tfirst, const int32_t* tn, const int64_t* chunk_items,
-                      const double2* tpart, double2* pnear, int nsm, cudaStream_t s) {
+                      const double2* tpart, int split, double2* pnear, int nsm, cudaStream_t s) {
   if (nchunk <= 0) return;
   const int grid = (int)std::min<int64_t>((nchunk + 3) / 4, (int64_t)nsm * 16);
-  k_p2p_items<<<grid, 128, 0, s>>>(nchunk, tfirst, tn, chunk_items, tpart, pnear);
+  k_p2p_items<<<grid, 128, 0, s>>>(nchunk, tfirst, tn, chunk_items, tpart, split, pnear);
 }
 
 void launch_p2p_sym(bool fp64, const DevPlan& dp, int64_t nwork, const int32_t* order, const int32_t* item_chunk,
                     const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst,
-                    const int32_t* sn, const int64_t* soff, const void* q, double2* tpart, void* scratch,
+                    const int32_t* sn, const int64_t* soff, const void* q, double2* tpart, void* scratch, int split,
                     unsigned long long* queue, int nsm, int blocks_per_sm, cudaStream_t s) {
   if (nwork <= 0) return;
   cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
-  const int grid = (int)std::min<int64_t>(nwork, (int64_t)nsm * std::max(1, std::min(blocks_per_sm, 64)));
+  const int grid = (int)std::min<int64_t>(nwork * split, (int64_t)nsm * std::max(1, std::min(blocks_per_sm, 64)));
   if (fp64)
     k_p2p_sym<false><<<grid, 128, 0, s>>>(dp, nwork, order, item_chunk, tfirst, tn, ptr, sfirst, sn, soff, q, tpart,
-                                          scratch, queue);
+                                          scratch, split, queue);
   else
     k_p2p_sym<true><<<grid, 128, 0, s>>>(dp, nwork, order, item_chunk, tfirst, tn, ptr, sfirst, sn, soff, q, tpart,
-                                         scratch, queue);
+                                         scratch, split, queue);
 }
 
 void launch_p2p_reduce(bool fp64, int64_t nleaf, const int32_t* first, const int32_t* n, const int64_t* rptr,
@@ -2859,40 +2818,45 @@ template <bool MIXED, int RB>
 static void p2p_rhs_go(const DevPlan& dp, int64_t nitem, const int32_t* order, const int32_t* item_chunk,
                        const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst,
                        const int32_t* sn, const void* q, int R, int r0, double2* pnear, double2* tpart,
-                       unsigned long long* queue, int grid, cudaStream_t s) {
+                       int split, unsigned long long* queue, int grid, cudaStream_t s) {
   k_p2p_rhs<MIXED, RB><<<grid, 128, P2PRhsCfg<MIXED, RB>::smem(), s>>>(dp, nitem, order, item_chunk, tfirst, tn, ptr,
-                                                                       sfirst, sn, q, R, r0, pnear, tpart, queue);
+                                                                       sfirst, sn, q, R, r0, pnear, tpart, split,
+                                                                       queue);
 }
 
 void launch_p2p_rhs(bool fp64, const DevPlan& dp, int64_t nitem, const int32_t* order, const int32_t* item_chunk,
                     const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst,
-                    const int32_t* sn, const void* q, int R, double2* pnear, double2* tpart,
+                    const int32_t* sn, const void* q, int R, double2* pnear, double2* tpart, int split,
                     unsigned long long* queue, int nsm, int blocks_per_sm, cudaStream_t s) {
   if (!nitem) return;
-  const int grid = (int)std::min<int64_t>(nitem, (int64_t)nsm * std::max(1, std::min(blocks_per_sm, 64)));
+  const int grid = (int)std::min<int64_t>(nitem * split, (int64_t)nsm * std::max(1, std::min(blocks_per_sm, 64)));
+  auto go = [&](auto rb, int r0) {
+    constexpr int RB = decltype(rb)::value;
+    cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
+    if (fp64)
+      p2p_rhs_go<false, RB>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, split,
+                            queue, grid, s);
+    else
+      p2p_rhs_go<true, RB>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, split,
+                           queue, grid, s);
+  };
   for (int r0 = 0; r0 < R;) {
     const int left = R - r0;
-    const int rb = left >= 8 ? 8 : (left >= 4 ? 4 : 1);
-    cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
-    if (rb == 8) {
-      if (fp64) p2p_rhs_go<false, 8>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, queue, grid, s);
-      else p2p_rhs_go<true, 8>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, queue, grid, s);
-    } else if (rb == 4) {
-      if (fp64) p2p_rhs_go<false, 4>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, queue, grid, s);
-      else p2p_rhs_go<true, 4>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, queue, grid, s);
-    } else {
-      if (fp64) p2p_rhs_go<false, 1>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, queue, grid, s);
-      else p2p_rhs_go<true, 1>(dp, nitem, order, item_chunk, tfirst, tn, ptr, sfirst, sn, q, R, r0, pnear, tpart, queue, grid, s);
-    }
+    const int rb = left >= 8 ? 8 : (left >= 4 ? 4 : left);
+    if (rb == 8) go(std::integral_constant<int, 8>(), r0);
+    if (rb == 4) go(std::integral_constant<int, 4>(), r0);
+    if (rb == 3) go(std::integral_constant<int, 3>(), r0);
+    if (rb == 2) go(std::integral_constant<int, 2>(), r0);
+    if (rb == 1) go(std::integral_constant<int, 1>(), r0);
     r0 += rb;
   }
 }
 
 void launch_p2p_items_rhs(int64_t nchunk, const int32_t* tfirst, const int32_t* tn, const int64_t* chunk_items,
-                          const double2* tpart, int R, double2* pnear, int nsm, cudaStream_t s) {
+                          const double2* tpart, int split, int R, double2* pnear, int nsm, cudaStream_t s) {
   if (nchunk <= 0) return;
   const int grid = (int)std::min<int64_t>((nchunk * 32 * R + 255) / 256, (int64_t)nsm * 16);
-  k_p2p_items_rhs<<<grid, 256, 0, s>>>(nchunk, tfirst, tn, chunk_items, tpart, R, pnear);
+  k_p2p_items_rhs<<<grid, 256, 0, s>>>(nchunk, tfirst, tn, chunk_items, tpart, split, R, pnear);
 }
 
 void launch_gather_rhs(bool fp64, const double2* qin, const int32_t* perm, void* q, int64_t n, int64_t stride, int R,

@@ -66,12 +66,16 @@ void launch_scatter(const double2* pnear, const double2* pfar, const int32_t* pe
 // decreasing work, `queue` is a device counter the launch resets.  With
 // item_chunk == nullptr items are chunks and sums are stored into pnear;
 // otherwise item partial sums go to tpart (32 per item) and
-// launch_p2p_items adds them per chunk, in item order.
+// launch_p2p_items adds them per chunk, in item order.  split > 1 (items with
+// item_chunk only): every item is cut into that many parts, part p taking
+// every split-th source tile from tile p on, with 32 sums of its own in
+// tpart ((item split + p) 32 ...).
 void launch_p2p(bool fp64, const DevPlan& dp, int64_t nitem, const int32_t* order, const int32_t* item_chunk,
                 const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst, const int32_t* sn,
-                const void* q, double2* pnear, double2* tpart, unsigned long long* queue, int nsm, cudaStream_t s);
+                const void* q, double2* pnear, double2* tpart, int split, unsigned long long* queue, int nsm,
+                cudaStream_t s);
 void launch_p2p_items(int64_t nchunk, const int32_t* tfirst, const int32_t* tn, const int64_t* chunk_items,
-                      const double2* tpart, double2* pnear, int nsm, cudaStream_t s);
+                      const double2* tpart, int split, double2* pnear, int nsm, cudaStream_t s);
 // Symmetric near field: symmetric blocks over items (k_p2p_sym: the target
 // side to tpart, the source side to scratch) and the per-leaf reduction of
 // the scratch into pnear (k_p2p_reduce).  Scratch holds double2 (fp64) or
@@ -80,7 +84,7 @@ void launch_p2p_items(int64_t nchunk, const int32_t* tfirst, const int32_t* tn, 
 void launch_p2p_sym(bool fp64, const DevPlan& dp, int64_t nwork, const int32_t* order, const int32_t* item_chunk,
                     const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst,
                     const int32_t* sn, const int64_t* soff, const void* q, double2* tpart, void* scratch,
-                    unsigned long long* queue, int nsm, int blocks_per_sm, cudaStream_t s);
+                    int split, unsigned long long* queue, int nsm, int blocks_per_sm, cudaStream_t s);
 void launch_p2p_reduce(bool fp64, int64_t nleaf, const int32_t* first, const int32_t* n, const int64_t* rptr,
                        const int64_t* roff, const void* scratch, double2* pnear, int nsm, cudaStream_t s);
 // Kernel attributes of the right-hand-side block kernels (call once per
@@ -101,10 +105,10 @@ void launch_l2p_tc(int L, const DevPlan& dp, const int32_t* leaves, int n, const
 // by launch_p2p_items_rhs.
 void launch_p2p_rhs(bool fp64, const DevPlan& dp, int64_t nitem, const int32_t* order, const int32_t* item_chunk,
                     const int32_t* tfirst, const int32_t* tn, const int64_t* ptr, const int32_t* sfirst,
-                    const int32_t* sn, const void* q, int R, double2* pnear, double2* tpart,
+                    const int32_t* sn, const void* q, int R, double2* pnear, double2* tpart, int split,
                     unsigned long long* queue, int nsm, int blocks_per_sm, cudaStream_t s);
 void launch_p2p_items_rhs(int64_t nchunk, const int32_t* tfirst, const int32_t* tn, const int64_t* chunk_items,
-                          const double2* tpart, int R, double2* pnear, int nsm, cudaStream_t s);
+                          const double2* tpart, int split, int R, double2* pnear, int nsm, cudaStream_t s);
 // q[i R + r] = qin[r stride + perm[i]] (zero for r >= nvec);
 // out[r stride + perm[i]] = pnear + pfar (r < nvec)
 void launch_gather_rhs(bool fp64, const double2* qin, const int32_t* perm, void* q, int64_t n, int64_t stride, int R,

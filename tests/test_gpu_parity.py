@@ -452,3 +452,21 @@ def test_near_field_target_remainders(ncrit, gpu):
     assert rel(ref, O.OracleFMM(p, p, 4, ncrit, 2 * np.pi * 2, -1).gemv(q)) <= FP64_TOL
     A.set_precision("mixed")
     assert rel(A.matvec(q), ref) <= MIXED_TOL
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 5, 7])
+def test_near_field_parts_and_block_widths(nrhs, gpu):
+    # few long near-field items, cut into parts (distinct sets: target-side
+    # kernels), for every number of right-hand sides per near-field launch
+    src, trg, L, ncrit, kappa = small_case("near_only")
+    A = make(src, trg, L, ncrit, kappa)
+    rng = np.random.default_rng(3)
+    Q = (rng.uniform(-1, 1, (nrhs, len(src))) + 1j * rng.uniform(-1, 1, (nrhs, len(src)))).astype(np.complex128)
+    d = np.linalg.norm(trg[:, None] - src[None], axis=-1)
+    ex = ((np.exp(1j * kappa * d) / (4 * np.pi * d)) @ Q.T).T
+    P = A.matvec(Q)
+    A.set_precision("mixed")
+    M = A.matvec(Q)
+    for r in range(nrhs):
+        assert rel(P[r], ex[r]) <= 1e-13
+        assert rel(M[r], ex[r]) <= MIXED_TOL

@@ -58,15 +58,6 @@ __device__ __forceinline__ typename cpx_t<T>::type ctw(int m) {
   }
   return r;
 }
-// acc += v * conj(w)
-template <typename C>
-__device__ __forceinline__ void cfmac(C& acc, C v, C w) {
-  acc.x = fma(v.x, w.x, acc.x);
-  acc.x = fma(v.y, w.y, acc.x);
-  acc.y = fma(v.y, w.x, acc.y);
-  acc.y = fma(-v.x, w.y, acc.y);
-}
-
 // ------------------------------------------------------------- gather/scatter
 template <typename T>
 __global__ void k_gather(const double2* __restrict__ qin, const int32_t* __restrict__ perm,
@@ -699,6 +690,40 @@ struct M2FCfg {
   static constexpr int NW = NW0 < 1 ? 1 : (NW0 > 8 ? 8 : NW0);
 };
 
+// One line of the forward DFT: out(k) = sum_a v[a] w^(k a), k < P = 2 L - 1,
+// a < L.  Outputs k and P - k are A - i B and A + i B with A = sum cos v,
+// B = sum sin v: 4 (L - 1) FMAs for the two instead of 8 (L - 1) for each.
+template <typename T, int L, typename C, typename Put>
+__device__ __forceinline__ void fdft_line(const C (&v)[L], Put put) {
+  constexpr int P = 2 * L - 1;
+  C s0 = v[0];
+#pragma unroll
+  for (int a = 1; a < L; a++) {
+    s0.x += v[a].x;
+    s0.y += v[a].y;
+  }
+  put(0, s0);
+#pragma unroll
+  for (int k = 1; k < L; k++) {
+    C A = v[0], B;
+#pragma unroll
+    for (int a = 1; a < L; a++) {
+      const C w = ctw<T, L>((k * a) % P);  // (cos, -sin)
+      A.x = fma(w.x, v[a].x, A.x);
+      A.y = fma(w.x, v[a].y, A.y);
+      B.x = a == 1 ? w.y * v[a].x : fma(w.y, v[a].x, B.x);  // -B
+      B.y = a == 1 ? w.y * v[a].y : fma(w.y, v[a].y, B.y);
+    }
+    C lo, hi;
+    lo.x = A.x - B.y;
+    lo.y = A.y + B.x;
+    hi.x = A.x + B.y;
+    hi.y = A.y - B.x;
+    put(k, lo);
+    put(P - k, hi);
+  }
+}
+
 template <typename T, int L>
 __global__ void __launch_bounds__(256) k_m2f(int64_t n, const typename cpx_t<T>::type* __restrict__ M,
                                              typename cpx_t<T>::type* __restrict__ F) {
@@ -741,13 +766,7 @@ __global__ void __launch_bounds__(256) k_m2f(int64_t n, const typename cpx_t<T>:
       C v[L];
 #pragma unroll
       for (int c = 0; c < L; c++) v[c] = Mi[ln * L + c];
-#pragma unroll
-      for (int k2 = 0; k2 < P; k2++) {
-        C acc = v[0];
-#pragma unroll
-        for (int c = 1; c < L; c++) cfma(acc, v[c], ctw<T, L>((k2 * c) % P));
-        A[ln * P + k2] = acc;
-      }
+      fdft_line<T, L>(v, [&](int k2, C o) { A[ln * P + k2] = o; });
     }
     __syncwarp();
     for (int ln = lane; ln < L * P; ln += 32) {  // axis 1: (a,k2) lines
@@ -755,26 +774,14 @@ __global__ void __launch_bounds__(256) k_m2f(int64_t n, const typename cpx_t<T>:
       C v[L];
 #pragma unroll
       for (int b = 0; b < L; b++) v[b] = A[(a * L + b) * P + k2];
-#pragma unroll
-      for (int k1 = 0; k1 < P; k1++) {
-        C acc = v[0];
-#pragma unroll
-        for (int b = 1; b < L; b++) cfma(acc, v[b], ctw<T, L>((k1 * b) % P));
-        B[(a * P + k1) * P + k2] = acc;
-      }
+      fdft_line<T, L>(v, [&](int k1, C o) { B[(a * P + k1) * P + k2] = o; });
     }
     __syncwarp();
     for (int ln = lane; ln < P * P; ln += 32) {  // axis 0: (k1,k2) lines
       C v[L];
 #pragma unroll
       for (int a = 0; a < L; a++) v[a] = B[a * P * P + ln];
-#pragma unroll
-      for (int k0 = 0; k0 < P; k0++) {
-        C acc = v[0];
-#pragma unroll
-        for (int a = 1; a < L; a++) cfma(acc, v[a], ctw<T, L>((k0 * a) % P));
-        F[e * PP + k0 * P * P + ln] = acc;
-      }
+      fdft_line<T, L>(v, [&](int k0, C o) { F[e * PP + k0 * P * P + ln] = o; });
     }
   }
 }
@@ -794,6 +801,51 @@ __global__ void k_permute_tables(int64_t n, int PP, const uint32_t* __restrict__
 }
 
 // -------------------------------------------------------------- M2L + F2L --
+// One line of the inverse DFT, pruned to its L low outputs:
+//   out[a] = sum_k v[k] conj(w)^(k a),  w = exp(-2 pi i / P), P = 2 L - 1.
+// The terms k and P - k share their cosine, and their sine up to its sign, so
+// they are added and subtracted first: 4 (L - 1) FMAs per output instead of
+// 8 (L - 1), none of them multiplications for a = 0.
+// One pair's share of one output, o += v_k conj(w) + v_(P-k) w (idft_line's
+// operations, for a thread that computes a single output).
+template <typename C>
+__device__ __forceinline__ void idft_pair(C& o, C vk, C vp, C w) {
+  o.x = fma(w.x, vk.x + vp.x, o.x);
+  o.y = fma(w.x, vk.y + vp.y, o.y);
+  o.x = fma(w.y, vk.y - vp.y, o.x);
+  o.y = fma(-w.y, vk.x - vp.x, o.y);
+}
+template <typename T, int L, typename C>
+__device__ __forceinline__ void idft_line(const C (&v)[2 * L - 1], C (&out)[L]) {
+  constexpr int P = 2 * L - 1;
+  C s[L], d[L];
+#pragma unroll
+  for (int k = 1; k < L; k++) {
+    s[k].x = v[k].x + v[P - k].x;
+    s[k].y = v[k].y + v[P - k].y;
+    d[k].x = v[k].x - v[P - k].x;
+    d[k].y = v[k].y - v[P - k].y;
+  }
+#pragma unroll
+  for (int a = 0; a < L; a++) {
+    C o = v[0];
+#pragma unroll
+    for (int k = 1; k < L; k++) {
+      if (a == 0) {
+        o.x += s[k].x;
+        o.y += s[k].y;
+      } else {
+        const C w = ctw<T, L>((k * a) % P);  // (cos, -sin)
+        o.x = fma(w.x, s[k].x, o.x);
+        o.y = fma(w.x, s[k].y, o.y);
+        o.x = fma(w.y, d[k].y, o.x);
+        o.y = fma(-w.y, d[k].x, o.y);
+      }
+    }
+    out[a] = o;
+  }
+}
+
 // Inverse DFT of one target slot's spectrum J (acc, K values per thread) into
 // its local expansion (fourier2geom, circulant.hpp:109-118):
 //   L_t[a,b,c] += (1/PP) sum_k J[k] conj(w)^(k0 a + k1 b + k2 c)
@@ -817,13 +869,10 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
     C v[PD];
 #pragma unroll
     for (int k0 = 0; k0 < PD; k0++) v[k0] = Js[k0 * PD * PD + ln];
+    C o[L];
+    idft_line<T, L>(v, o);
 #pragma unroll
-    for (int a = 0; a < L; a++) {
-      C s = v[0];
-#pragma unroll
-      for (int k0 = 1; k0 < PD; k0++) cfmac(s, v[k0], ctw<T, L>((k0 * a) % PD));
-      Cb[a * PD * PD + ln] = s;
-    }
+    for (int a = 0; a < L; a++) Cb[a * PD * PD + ln] = o[a];
   }
   __syncthreads();
   for (int ln = threadIdx.x; ln < L * PD; ln += NT) {  // axis 1: (a,k2) lines -> b
@@ -831,27 +880,23 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
     C v[PD];
 #pragma unroll
     for (int k1 = 0; k1 < PD; k1++) v[k1] = Cb[(a * PD + k1) * PD + k2];
+    C o[L];
+    idft_line<T, L>(v, o);
 #pragma unroll
-    for (int b = 0; b < L; b++) {
-      C s = v[0];
-#pragma unroll
-      for (int k1 = 1; k1 < PD; k1++) cfmac(s, v[k1], ctw<T, L>((k1 * b) % PD));
-      D[(a * L + b) * PD + k2] = s;
-    }
+    for (int b = 0; b < L; b++) D[(a * L + b) * PD + k2] = o[b];
   }
   __syncthreads();
   for (int ln = threadIdx.x; ln < L * L; ln += NT) {  // axis 2: (a,b) lines -> c
     C v[PD];
 #pragma unroll
     for (int k2 = 0; k2 < PD; k2++) v[k2] = D[ln * PD + k2];
+    C s[L];
+    idft_line<T, L>(v, s);
 #pragma unroll
     for (int c = 0; c < L; c++) {
-      C s = v[0];
-#pragma unroll
-      for (int k2 = 1; k2 < PD; k2++) cfmac(s, v[k2], ctw<T, L>((k2 * c) % PD));
       C o = Lt[ln * L + c];
-      o.x += s.x * inv;
-      o.y += s.y * inv;
+      o.x += s[c].x * inv;
+      o.y += s[c].y * inv;
       Lt[ln * L + c] = o;
     }
   }
@@ -885,13 +930,10 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
     C v[PD];
 #pragma unroll
     for (int k0 = 0; k0 < PD; k0++) v[k0] = J[k0 * PD * PD + ln];
+    C o[L];
+    idft_line<T, L>(v, o);
 #pragma unroll
-    for (int a = 0; a < L; a++) {
-      C s = v[0];
-#pragma unroll
-      for (int k0 = 1; k0 < PD; k0++) cfmac(s, v[k0], ctw<T, L>((k0 * a) % PD));
-      Cq[a * PD * PD + ln] = s;
-    }
+    for (int a = 0; a < L; a++) Cq[a * PD * PD + ln] = o[a];
   }
   __syncthreads();
   for (int x = threadIdx.x; x < RB * L * PD; x += NT) {  // axis 1: (a,k2) lines -> b
@@ -902,13 +944,10 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
     C v[PD];
 #pragma unroll
     for (int k1 = 0; k1 < PD; k1++) v[k1] = Cq[(a * PD + k1) * PD + k2];
+    C o[L];
+    idft_line<T, L>(v, o);
 #pragma unroll
-    for (int b = 0; b < L; b++) {
-      C s = v[0];
-#pragma unroll
-      for (int k1 = 1; k1 < PD; k1++) cfmac(s, v[k1], ctw<T, L>((k1 * b) % PD));
-      Dq[(a * L + b) * PD + k2] = s;
-    }
+    for (int b = 0; b < L; b++) Dq[(a * L + b) * PD + k2] = o[b];
   }
   __syncthreads();
   for (int x = threadIdx.x; x < RB * L * L; x += NT) {  // axis 2: (a,b) lines -> c
@@ -918,14 +957,13 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
     C v[PD];
 #pragma unroll
     for (int k2 = 0; k2 < PD; k2++) v[k2] = Dq[ln * PD + k2];
+    C s[L];
+    idft_line<T, L>(v, s);
 #pragma unroll
     for (int c = 0; c < L; c++) {
-      C s = v[0];
-#pragma unroll
-      for (int k2 = 1; k2 < PD; k2++) cfmac(s, v[k2], ctw<T, L>((k2 * c) % PD));
       C o = Lq[ln * L + c];
-      o.x += s.x * inv;
-      o.y += s.y * inv;
+      o.x += s[c].x * inv;
+      o.y += s[c].y * inv;
       Lq[ln * L + c] = o;
     }
   }
@@ -1465,7 +1503,7 @@ __global__ void __launch_bounds__(M2LBulk<L>::NT, M2LBulk<L>::CTAS) k_m2l_bulk(
         const float2* v = Js + sp * PP + ln;
         float2 sum = v[0];
 #pragma unroll
-        for (int k0 = 1; k0 < PD; k0++) cfmac(sum, v[k0 * PD * PD], tw[(k0 * a) % PD]);
+        for (int k0 = 1; k0 < L; k0++) idft_pair(sum, v[k0 * PD * PD], v[(PD - k0) * PD * PD], tw[(k0 * a) % PD]);
         Cb[sp * L * PD * PD + a * PD * PD + ln] = sum;
       }
       if (!(ok = cbarrier())) continue;
@@ -1476,7 +1514,7 @@ __global__ void __launch_bounds__(M2LBulk<L>::NT, M2LBulk<L>::CTAS) k_m2l_bulk(
         const float2* v = Cb + sp * L * PD * PD + a * PD * PD + k2;
         float2 sum = v[0];
 #pragma unroll
-        for (int k1 = 1; k1 < PD; k1++) cfmac(sum, v[k1 * PD], tw[(k1 * b) % PD]);
+        for (int k1 = 1; k1 < L; k1++) idft_pair(sum, v[k1 * PD], v[(PD - k1) * PD], tw[(k1 * b) % PD]);
         D[sp * L * L * PD + (a * L + b) * PD + k2] = sum;
       }
       if (!(ok = cbarrier())) continue;
@@ -1486,7 +1524,7 @@ __global__ void __launch_bounds__(M2LBulk<L>::NT, M2LBulk<L>::CTAS) k_m2l_bulk(
         const float2* v = D + sp * L * L * PD + ln * PD;
         float2 sum = v[0];
 #pragma unroll
-        for (int k2 = 1; k2 < PD; k2++) cfmac(sum, v[k2], tw[(k2 * c) % PD]);
+        for (int k2 = 1; k2 < L; k2++) idft_pair(sum, v[k2], v[(PD - k2)], tw[(k2 * c) % PD]);
         lold.x += sum.x * inv;
         lold.y += sum.y * inv;
         *l3 = lold;

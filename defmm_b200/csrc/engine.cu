@@ -15,6 +15,7 @@
 #include "../../include/defmm_b200.h"
 #include "engine_internal.h"
 #include "fmm_kernels.h"
+#include "m2l_lists.hpp"
 #include "plan.hpp"
 #include "plan_device.hpp"
 
@@ -73,6 +74,11 @@ struct defmm_handle {
   // precision-dependent arrays
   DevBuf M, Lx, F, q, sig, sig2, ptab;
   const uint32_t* d_ptab_key = nullptr;
+  // M2L lists compacted (device_m2l_lists): per level and cone, the listed
+  // target / source slots before it; m2l_ranked: the device entries hold
+  // positions in DevPlan::m2l_slist
+  std::vector<std::vector<int64_t>> tU, sU;
+  bool m2l_ranked = false;
   int64_t f_cap = 0;  // source slots per F batch buffer
   // FP64 vectors
   DevBuf pnear, pfar, qin, out, chk;
@@ -473,6 +479,41 @@ int upload_plan(defmm_handle* h) {
   if ((st = ensure(h, h->pnear, 16 * nT)) || (st = ensure(h, h->pfar, 16 * nT)) ||
       (st = ensure(h, h->qin, 16 * nS)) || (st = ensure(h, h->out, 16 * nT)))
     return st;
+  {  // target slots with a list, source slots in some list; entries renumbered
+     // to the latter (last: an upload that failed before can be repeated)
+    const size_t nT1 = (size_t)p.sT.n + 1, bytes = nT1 * 8 + nT1 * 4 + (size_t)(p.sS.n + 1) * 4;
+    void* cp = nullptr;
+    CK(cudaMalloc(&cp, bytes));
+    h->plan_allocs.push_back(cp);
+    h->dev_bytes += bytes;
+    int64_t* cptr = static_cast<int64_t*>(cp);
+    int32_t* tl = reinterpret_cast<int32_t*>(cptr + nT1);
+    int32_t* sl = tl + nT1;
+    std::vector<int64_t> atT, atS;
+    for (int l = 0; l < p.lv.nlvl; l++) {
+      atT.insert(atT.end(), p.sT.cone_begin[l].begin(), p.sT.cone_begin[l].end());
+      atS.insert(atS.end(), p.sS.cone_begin[l].begin(), p.sS.cone_begin[l].end());
+    }
+    std::string e;
+    const int64_t nent = p.m2l_ptr.empty() ? 0 : p.m2l_ptr.back();
+    st = dfb::device_m2l_lists(d.m2l_ptr, const_cast<int32_t*>(d.m2l_src), nent, p.sT.n, p.sS.n, atT, atS, cptr, tl,
+                               sl, e);
+    if (st) return h->fail(st == -5 ? DEFMM_ERR_MEMORY : DEFMM_ERR_CUDA, e);
+    h->m2l_ranked = true;
+    d.m2l_cptr = cptr;
+    d.m2l_tlist = tl;
+    d.m2l_slist = sl;
+    h->tU.assign(p.lv.nlvl, {});
+    h->sU.assign(p.lv.nlvl, {});
+    size_t a = 0, b = 0;
+    for (int l = 0; l < p.lv.nlvl; l++) {
+      const size_t na = p.sT.cone_begin[l].size(), nb = p.sS.cone_begin[l].size();
+      h->tU[l].assign(atT.begin() + a, atT.begin() + a + na);
+      h->sU[l].assign(atS.begin() + b, atS.begin() + b + nb);
+      a += na;
+      b += nb;
+    }
+  }
   return 0;
 }
 
@@ -846,14 +887,17 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
     for (int l = p.lv.max_stage; l < nl && h->tune_m2l; l++) {
       for (int c = 0; c < 4; c++) h->tune_ms[l][c] = h->tune_pairs[l][c] = 0;
       if (!h->tune_lvl_on[l]) continue;
-      const auto& cS = p.sS.cone_begin[l];
-      const auto& cT = p.sT.cone_begin[l];
+      const auto& cS = h->sU[l];
+      const auto& cT = h->tU[l];
       const int nc = (int)cS.size() - 1;
       for (int c0 = 0; c0 < nc;) {
         int c1 = c0 + 1;
         while (c1 < nc && cS[c1 + 1] - cS[c0] <= h->f_cap) c1++;
         const int64_t fs0 = cS[c0], fs1 = cS[c1], ts0 = cT[c0], ts1 = cT[c1];
         constexpr int kSlices = 16;
+        int64_t ent[kSlices + 1] = {0};  // list entries before each slice
+        for (int i = 0; i <= kSlices && ts1 > ts0 && fs1 > fs0; i++)
+          CK(cudaMemcpy(&ent[i], d.m2l_cptr + ts0 + (ts1 - ts0) * i / kSlices, 8, cudaMemcpyDeviceToHost));
         for (int i = 0; i < kSlices && ts1 > ts0 && fs1 > fs0; i++) {
           const int64_t a0 = ts0 + (ts1 - ts0) * i / kSlices, a1 = ts0 + (ts1 - ts0) * (i + 1) / kSlices;
           if (a1 <= a0) continue;
@@ -868,7 +912,7 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
           cudaEventElapsedTime(&a, h->ev[2 * PH_M2L], h->ev[2 * PH_M2L + 1]);
           tm2l += a;
           h->tune_ms[l][c] += a;
-          h->tune_pairs[l][c] += (double)(p.m2l_ptr[a1] - p.m2l_ptr[a0]);
+          h->tune_pairs[l][c] += (double)(ent[i + 1] - ent[i]);
         }
         c0 = c1;
       }
@@ -902,8 +946,8 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
   float tm2f = 0, tm2l = 0, tl2l = 0;
   const size_t cs = fp64 ? 16 : 8;
   for (int l = p.lv.max_stage; l < nl; l++) {
-    const auto& cS = p.sS.cone_begin[l];
-    const auto& cT = p.sT.cone_begin[l];
+    const auto& cS = h->sU[l];
+    const auto& cT = h->tU[l];
     const int nc = (int)cS.size() - 1;
     int c0 = 0;
     while (c0 < nc) {
@@ -912,7 +956,7 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
       const int64_t fs0 = cS[c0], fs1 = cS[c1], ts0 = cT[c0], ts1 = cT[c1];
       if (ts1 > ts0 && fs1 > fs0) {
         rec(h, 2 * PH_M2F);
-        ops->m2f(fs1 - fs0, (const char*)h->M.p + fs0 * p.LL * cs, h->F.p, sf);
+        ops->m2f(fs1 - fs0, 1, d.m2l_slist + fs0, h->M.p, h->F.p, sf);
         nl_ += 2;
         rec(h, 2 * PH_M2F + 1);
         rec(h, 2 * PH_M2L);
@@ -1071,8 +1115,9 @@ int run_gemv_grouped(defmm_handle* h, const double2* qin, int64_t stride_in, dou
   const int lf = g.lh < 0 ? 0 : g.lh + 1;  // first LF level
   // M2F + M2L of source cones [c0, c1) at level l: targets into Lbase
   auto far_cones = [&](int l, int64_t c0, int64_t c1, void* Mbase, void* Lbase) -> int {
-    const auto& cS = p.sS.cone_begin[l];
-    const auto& cT = p.sT.cone_begin[l];
+    const auto& cS = h->sU[l];  // listed slots before each cone
+    const auto& cT = h->tU[l];
+    const auto& aT = p.sT.cone_begin[l];
     int64_t a = c0;
     while (a < c1) {
       int64_t b = a + 1;
@@ -1080,7 +1125,7 @@ int run_gemv_grouped(defmm_handle* h, const double2* qin, int64_t stride_in, dou
       const int64_t fs0 = cS[a], fs1 = cS[b], ts0 = cT[a], ts1 = cT[b];
       if (ts1 > ts0 && fs1 > fs0) {
         timed(PH_M2F, [&] {
-          ops->m2f((fs1 - fs0) * R, (const char*)Mbase + (size_t)fs0 * slot_b, g.F.p, s);
+          ops->m2f(fs1 - fs0, R, d.m2l_slist + fs0, Mbase, g.F.p, s);
         });
         timed(PH_M2L, [&] {
           if (R == 1) {
@@ -1088,7 +1133,7 @@ int run_gemv_grouped(defmm_handle* h, const double2* qin, int64_t stride_in, dou
             m2l_choice(h, pi, l, &nt_l, &pair_l);
             ops->m2l(d, ts0, ts1, fs0, fs1, g.F.p, h->ptab.p, Lbase, h->d_queue + 1, h->nsm, nt_l, pair_l, s);
           } else
-            ops->m2l_rhs(d, ts0, ts1, fs0, fs1, R, h->rhs_block_m2l, g.F.p, h->ptab.p, Lbase, h->d_queue + 1,
+            ops->m2l_rhs(d, ts0, ts1, aT[a], aT[b], fs0, fs1, R, h->rhs_block_m2l, g.F.p, h->ptab.p, Lbase, h->d_queue + 1,
                          h->nsm, h->m2l_staging ? h->m2l_lgroup : 0, s);
         });
         nk += 2;
@@ -1609,6 +1654,7 @@ int defmm_prcmpt(defmm_handle* h, int L, int Ncrit, double kappa, int lvMAX) {
   h->built = false;
   h->uploaded = false;
   h->plan = Plan();
+  h->m2l_ranked = false;
   h->plan.keep_lists = h->keep_lists;
   std::string e;
   // the level walk on the GPU when there is one (list records for parity
@@ -1997,10 +2043,10 @@ int defmm_info(const defmm_handle* h, int what, int64_t* v) {
       *v = n;
       break;
     }
-    case DEFMM_INFO_M2F_SLOTS: {  // source slots at precomputed levels that have target slots in their cone
+    case DEFMM_INFO_M2F_SLOTS: {  // source slots in some M2L list; before the upload, those with target slots in their cone
       int64_t n = 0;
       for (int l = 0; l < p.lv.nlvl; l++) {
-        const auto& cS = p.sS.cone_begin[l];
+        const auto& cS = h->uploaded ? h->sU[l] : p.sS.cone_begin[l];
         const auto& cT = p.sT.cone_begin[l];
         for (size_t c = 0; c + 1 < cS.size() && c + 1 < cT.size(); c++)
           if (cT[c + 1] > cT[c]) n += cS[c + 1] - cS[c];
@@ -2083,6 +2129,15 @@ int defmm_dump_m2l(const defmm_handle* h, int64_t* ptr, int32_t* src, uint32_t* 
   } else {
     if (src) std::memcpy(src, p.m2l_src.data(), p.m2l_src.size() * 4);
     if (tab) std::memcpy(tab, p.m2l_tab.data(), p.m2l_tab.size() * 4);
+  }
+  if (src && p.dev_m2l_src && h->m2l_ranked) {  // positions -> source slots
+    std::vector<int32_t> sl((size_t)p.sS.n);
+    if (!sl.empty() &&
+        cudaMemcpy(sl.data(), h->dp.m2l_slist, sl.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
+      cudaGetLastError();
+      return DEFMM_ERR_CUDA;
+    }
+    for (int64_t i = 0; i < n[1]; i++) src[i] = sl[src[i]];
   }
   if (tab)  // ids -> (table << 6) | hash keys
     for (int64_t i = 0; i < n[1]; i++) tab[i] = p.ptab_key[tab[i]];

@@ -6,6 +6,7 @@
 #include "ptx.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <mutex>
 #include <set>
 #include <type_traits>
@@ -725,7 +726,8 @@ __device__ __forceinline__ void fdft_line(const C (&v)[L], Put put) {
 }
 
 template <typename T, int L>
-__global__ void __launch_bounds__(256) k_m2f(int64_t n, const typename cpx_t<T>::type* __restrict__ M,
+__global__ void __launch_bounds__(256) k_m2f(int64_t n, int R, const int32_t* __restrict__ slist,
+                                             const typename cpx_t<T>::type* __restrict__ M,
                                              typename cpx_t<T>::type* __restrict__ F) {
   typedef typename cpx_t<T>::type C;
   constexpr int P = 2 * L - 1, LL = L * L * L, PP = P * P * P;
@@ -740,11 +742,14 @@ __global__ void __launch_bounds__(256) k_m2f(int64_t n, const typename cpx_t<T>:
   constexpr int NV = (LL + 31) / 32;
   const int64_t e0 = (int64_t)blockIdx.x * NW + warp, de = (int64_t)gridDim.x * NW;
   C nx[NV];
+  // expansion e: right-hand side e mod R of the (e / R)-th listed slot
+  auto row = [&](int64_t e) { return M + ((int64_t)slist[e / R] * R + e % R) * LL; };
   if (e0 < n) {
+    const C* Me = row(e0);
 #pragma unroll
     for (int m = 0; m < NV; m++) {
       const int i = lane + 32 * m;
-      nx[m] = i < LL ? M[e0 * LL + i] : czero<C>();
+      nx[m] = i < LL ? Me[i] : czero<C>();
     }
   }
   for (int64_t e = e0; e < n; e += de) {
@@ -756,10 +761,11 @@ __global__ void __launch_bounds__(256) k_m2f(int64_t n, const typename cpx_t<T>:
     }
     __syncwarp();
     if (e + de < n) {
+      const C* Me = row(e + de);
 #pragma unroll
       for (int m = 0; m < NV; m++) {
         const int i = lane + 32 * m;
-        if (i < LL) nx[m] = M[(e + de) * LL + i];
+        if (i < LL) nx[m] = Me[i];
       }
     }
     for (int ln = lane; ln < L * L; ln += 32) {  // axis 2: (a,b) lines
@@ -852,10 +858,11 @@ __device__ __forceinline__ void idft_line(const C (&v)[2 * L - 1], C (&out)[L]) 
 // pruned to a,b,c < L, one line per thread per axis pass in shared memory.
 // Safe to call twice in a row: each pass reads only what the previous pass
 // wrote after the barrier between them.
-template <typename T, int L, int NT>
+// a() and b() run after the first and the second barrier.
+template <typename T, int L, int NT, typename HookA, typename HookB>
 __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, typename cpx_t<T>::type* Js,
                                         typename cpx_t<T>::type* Cb, typename cpx_t<T>::type* D,
-                                        typename cpx_t<T>::type* __restrict__ Lt) {
+                                        typename cpx_t<T>::type* __restrict__ Lt, HookA hook_a, HookB hook_b) {
   typedef typename cpx_t<T>::type C;
   constexpr int PD = 2 * L - 1, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   const T inv = T(1) / T(PP);
@@ -865,6 +872,7 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
     if (i < PP) Js[i] = acc[k];
   }
   __syncthreads();
+  hook_a();
   for (int ln = threadIdx.x; ln < PD * PD; ln += NT) {  // axis 0: (k1,k2) lines -> a
     C v[PD];
 #pragma unroll
@@ -875,6 +883,7 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
     for (int a = 0; a < L; a++) Cb[a * PD * PD + ln] = o[a];
   }
   __syncthreads();
+  hook_b();
   for (int ln = threadIdx.x; ln < L * PD; ln += NT) {  // axis 1: (a,k2) lines -> b
     const int a = ln / PD, k2 = ln % PD;
     C v[PD];
@@ -907,10 +916,10 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
 // axis pass runs over the lines of all RB spectra, so the CTA's threads stay
 // busy and the transform takes three barriers instead of 3 RB.  Every
 // output is computed by the operations of m2l_f2l for its spectrum.
-template <typename T, int L, int NT, int RB>
+template <typename T, int L, int NT, int RB, typename HookA, typename HookB>
 __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, typename cpx_t<T>::type* Js,
                                             typename cpx_t<T>::type* Cb, typename cpx_t<T>::type* D,
-                                            typename cpx_t<T>::type* __restrict__ Lt) {
+                                            typename cpx_t<T>::type* __restrict__ Lt, HookA hook_a, HookB hook_b) {
   typedef typename cpx_t<T>::type C;
   constexpr int PD = 2 * L - 1, PP = PD * PD * PD, K = (PP + NT - 1) / NT, LL = L * L * L;
   constexpr int NB = L * PD * PD, ND = L * L * PD;  // per spectrum: Cb, D elements
@@ -923,6 +932,7 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
       for (int b = 0; b < RB; b++) Js[b * PP + i] = acc[k * RB + b];
   }
   __syncthreads();
+  hook_a();
   for (int x = threadIdx.x; x < RB * PD * PD; x += NT) {  // axis 0: (k1,k2) lines -> a
     const int b = x / (PD * PD), ln = x % (PD * PD);
     const C* J = Js + b * PP;
@@ -936,6 +946,7 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
     for (int a = 0; a < L; a++) Cq[a * PD * PD + ln] = o[a];
   }
   __syncthreads();
+  hook_b();
   for (int x = threadIdx.x; x < RB * L * PD; x += NT) {  // axis 1: (a,k2) lines -> b
     const int r = x / (L * PD), ln = x % (L * PD);
     const int a = ln / PD, k2 = ln % PD;
@@ -969,129 +980,210 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
   }
 }
 
-// One CTA per target slot of a cone batch (M2L.hpp:115-157 target-stationary,
-// then the inverse DFT above):
+// Work queue of the M2L kernels: CTAs take work items in order (so the target
+// slots in flight stay a contiguous window of one cone, and F_s and U_k are
+// served from L2) and fetch the next item's index and lists while the
+// current item's inverse DFTs run, so that an item starts with its spectra
+// loads instead of a chain of three misses (index, pointers, entries).
+// NL lists per item, for up to kCap entries each (the rest is read directly).
+template <int NL, int NT>
+struct M2LQueue {
+  static constexpr int kCap = NT / NL < 64 ? NT / NL : 64;
+  struct Shared {
+    int64_t item[2], eb[2][NL];
+    int len[2][NL];
+    int2 e[2][NL][kCap];  // (position in the F batch's list, permuted spectrum)
+  };
+  Shared& sh;
+  const DevPlan& P;
+  unsigned long long* queue;
+  int64_t nwork;
+  int64_t b = 0, fetched = 0;
+  int n = 0;
+  int2 my;
+  __device__ __forceinline__ M2LQueue(Shared& s, const DevPlan& p, unsigned long long* q, int64_t nw)
+      : sh(s), P(p), queue(q), nwork(nw) {}
+  // every thread: list j's entry i of the next item
+  __device__ __forceinline__ int j() const { return threadIdx.x / kCap; }
+  __device__ __forceinline__ int i() const { return threadIdx.x % kCap; }
+  __device__ __forceinline__ void fetch() {
+    if (threadIdx.x == 0) fetched = gridDim.x + (int64_t)atomicAdd(queue, 1ULL);
+  }
+  // the CTA's first item, without the queue; then a barrier
+  __device__ __forceinline__ void first(int64_t u, int64_t u1) {
+    fetched = blockIdx.x;
+    publish(0);
+    pointers(fetched, u, u1);
+    entries();
+    store(0);
+  }
+  __device__ __forceinline__ void publish(int ph) {  // before a barrier
+    if (threadIdx.x == 0) sh.item[ph] = fetched;
+  }
+  // after that barrier: pointers of listed target slot u + j (none at or past u1)
+  __device__ __forceinline__ void pointers(int64_t item, int64_t u, int64_t u1) {
+    n = 0;
+    if (j() < NL && item < nwork && u + j() < u1) {
+      b = P.m2l_cptr[u + j()];
+      n = (int)(P.m2l_cptr[u + j() + 1] - b);
+    }
+  }
+  __device__ __forceinline__ void entries() {
+    if (i() < n) my = make_int2(P.m2l_src[b + i()], (int)P.m2l_tab[b + i()]);
+  }
+  __device__ __forceinline__ void store(int ph) {  // then a barrier
+    if (j() >= NL) return;
+    if (i() < n) sh.e[ph][j()][i()] = my;
+    if (i() == 0) {
+      sh.eb[ph][j()] = b;
+      sh.len[ph][j()] = n;
+    }
+  }
+  // entry x of list jj of the current item, from memory
+  __device__ __forceinline__ int2 direct(int ph, int jj, int x) const {
+    const int64_t g = sh.eb[ph][jj] + x;
+    return make_int2(P.m2l_src[g], (int)P.m2l_tab[g]);
+  }
+};
+
+// One CTA per listed target slot [u0, u1) of a cone batch (M2L.hpp:115-157
+// target-stationary, then the inverse DFT above):
 //   J[i] = sum_{(s, k) in list(t)} U_k[i] F_s[i]          (registers)
 // J never leaves the SM.
 template <typename T, int L, int NT>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(DevPlan P, int64_t t0, int64_t t1, int64_t f0, int64_t f1,
+__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
                                                        const typename cpx_t<T>::type* __restrict__ F,
                                                        const typename cpx_t<T>::type* __restrict__ ptab,
                                                        typename cpx_t<T>::type* __restrict__ Lx,
                                                        unsigned long long* __restrict__ queue) {
   typedef typename cpx_t<T>::type C;
+  typedef M2LQueue<1, NT> Q;
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Js = reinterpret_cast<C*>(smem_raw);
   C* Cb = Js + PP;
   C* D = Cb + L * PD * PD;
-  __shared__ int64_t cur;
-  // target slots are taken in order from a queue, so the slots in flight
-  // stay a contiguous window of one cone (good L2 reuse of F and U)
-  for (;;) {
-    __syncthreads();  // the previous slot's inverse DFT is done with Js/Cb/D
-    if (threadIdx.x == 0) cur = t0 + (int64_t)atomicAdd(queue, 1ULL);
-    __syncthreads();
-    const int64_t t = cur;
-    if (t >= t1) break;
-    const int64_t eb = P.m2l_ptr[t], ee = P.m2l_ptr[t + 1];
+  __shared__ typename Q::Shared qs;
+  Q q(qs, P, queue, u1 - u0);
+  q.first(u0 + (int64_t)blockIdx.x, u1);
+  __syncthreads();
+  for (int ph = 0; qs.item[ph] < u1 - u0; ph ^= 1) {
+    q.fetch();
+    const int64_t t = P.m2l_tlist[u0 + qs.item[ph]];
+    const int n = qs.len[ph][0];
     C acc[K];
 #pragma unroll
     for (int k = 0; k < K; k++) acc[k] = czero<C>();
-#pragma unroll 2
-    for (int64_t e = eb; e < ee; e++) {
-      const int64_t src = P.m2l_src[e];
-      if (src < f0 || src >= f1) {  // entry outside this cone batch: a plan bug
+    auto add = [&](int2 e) {
+      if (e.x < f0 || e.x >= f1) {  // entry outside this cone batch: a plan bug
         if (threadIdx.x == 0) atomicExch(P.err, 1);
-        continue;
+        return;
       }
-      const C* Fs = F + (src - f0) * PP;
-      const C* U = ptab + (int64_t)P.m2l_tab[e] * PP;
+      const C* Fs = F + (e.x - f0) * PP;
+      const C* U = ptab + (int64_t)(uint32_t)e.y * PP;
 #pragma unroll
       for (int k = 0; k < K; k++) {
         const int i = threadIdx.x + k * NT;
         if (i < PP) cfma(acc[k], __ldg(U + i), __ldg(Fs + i));
       }
-    }
-    m2l_f2l<T, L, NT>(acc, Js, Cb, D, Lx + t * LL);
+    };
+    const int ns = min(n, Q::kCap);
+#pragma unroll 2
+    for (int x = 0; x < ns; x++) add(qs.e[ph][0][x]);
+    for (int x = ns; x < n; x++) add(q.direct(ph, 0, x));
+    q.publish(ph ^ 1);
+    m2l_f2l<T, L, NT>(acc, Js, Cb, D, Lx + t * LL, [&] { q.pointers(qs.item[ph ^ 1], u0 + qs.item[ph ^ 1], u1); },
+                      [&] { q.entries(); });
+    q.store(ph ^ 1);
+    __syncthreads();
   }
 }
 
-// Two consecutive target slots per CTA.  Each slot's list is sorted by
+// Two consecutive listed target slots per CTA.  Each slot's list is sorted by
 // source slot, so a merge of the two lists finds their common sources
 // (about a third of the pairs at order 5), whose spectrum F_s is then read
 // once for both.  Every accumulator sees its own list in list order with the
 // same operations as k_m2l, so the results are bit-identical to it.
 template <typename T, int L, int NT>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_pair(DevPlan P, int64_t t0, int64_t t1, int64_t f0, int64_t f1,
+__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_pair(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
                                                             const typename cpx_t<T>::type* __restrict__ F,
                                                             const typename cpx_t<T>::type* __restrict__ ptab,
                                                             typename cpx_t<T>::type* __restrict__ Lx,
                                                             unsigned long long* __restrict__ queue) {
   typedef typename cpx_t<T>::type C;
+  typedef M2LQueue<2, NT> Q;
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Js = reinterpret_cast<C*>(smem_raw);
   C* Cb = Js + PP;
   C* D = Cb + L * PD * PD;
-  __shared__ int64_t cur;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) cur = t0 + 2 * (int64_t)atomicAdd(queue, 1ULL);
-    __syncthreads();
-    const int64_t t = cur;
-    if (t >= t1) break;
-    const bool two = t + 1 < t1;
-    int64_t a = P.m2l_ptr[t], b = P.m2l_ptr[t + 1];
-    const int64_t ae = b, be = two ? P.m2l_ptr[t + 2] : b;
+  __shared__ typename Q::Shared qs;
+  const int64_t nwork = (u1 - u0 + 1) / 2;
+  Q q(qs, P, queue, nwork);
+  q.first(u0 + 2 * (int64_t)blockIdx.x, u1);
+  __syncthreads();
+  for (int ph = 0; qs.item[ph] < nwork; ph ^= 1) {
+    q.fetch();
+    const int64_t u = u0 + 2 * qs.item[ph];
+    const bool two = u + 1 < u1;
+    const int64_t t = P.m2l_tlist[u], t2 = P.m2l_tlist[two ? u + 1 : u];
+    const int ae = qs.len[ph][0], be = qs.len[ph][1];
     C acc0[K], acc1[K];
 #pragma unroll
     for (int k = 0; k < K; k++) acc0[k] = acc1[k] = czero<C>();
-    while (a < ae || b < be) {
-      const int64_t sa = a < ae ? (int64_t)P.m2l_src[a] : INT64_MAX;
-      const int64_t sb = b < be ? (int64_t)P.m2l_src[b] : INT64_MAX;
-      const int64_t src = sa < sb ? sa : sb;
-      if (src < f0 || src >= f1) {  // entry outside this cone batch: a plan bug
-        if (threadIdx.x == 0) atomicExch(P.err, 1);
-        if (sa == src) a++;
-        if (sb == src) b++;
-        continue;
-      }
-      const C* Fs = F + (src - f0) * PP;
-      if (sa == sb) {
-        const C* U0 = ptab + (int64_t)P.m2l_tab[a] * PP;
-        const C* U1 = ptab + (int64_t)P.m2l_tab[b] * PP;
+    const int2 none = make_int2(INT_MAX, 0);
+    // the merge over entries at(list, x)
+    auto merge = [&](auto at) {
+      int a = 0, b = 0;
+      int2 ea = a < ae ? at(0, a) : none, eb = b < be ? at(1, b) : none;
+      while (a < ae || b < be) {
+        const int src = ea.x < eb.x ? ea.x : eb.x;
+        const bool ha = ea.x == src, hb = eb.x == src;
+        const int ka = ea.y, kb = eb.y;
+        if (ha) ea = ++a < ae ? at(0, a) : none;
+        if (hb) eb = ++b < be ? at(1, b) : none;
+        if (src < f0 || src >= f1) {  // entry outside this cone batch: a plan bug
+          if (threadIdx.x == 0) atomicExch(P.err, 1);
+          continue;
+        }
+        const C* Fs = F + (src - f0) * PP;
+        const C* U0 = ptab + (int64_t)(uint32_t)ka * PP;
+        const C* U1 = ptab + (int64_t)(uint32_t)kb * PP;
+        if (ha && hb) {
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-          const int i = threadIdx.x + k * NT;
-          if (i < PP) {
-            const C f = __ldg(Fs + i);
-            cfma(acc0[k], __ldg(U0 + i), f);
-            cfma(acc1[k], __ldg(U1 + i), f);
+          for (int k = 0; k < K; k++) {
+            const int i = threadIdx.x + k * NT;
+            if (i < PP) {
+              const C f = __ldg(Fs + i);
+              cfma(acc0[k], __ldg(U0 + i), f);
+              cfma(acc1[k], __ldg(U1 + i), f);
+            }
+          }
+        } else if (ha) {
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const int i = threadIdx.x + k * NT;
+            if (i < PP) cfma(acc0[k], __ldg(U0 + i), __ldg(Fs + i));
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const int i = threadIdx.x + k * NT;
+            if (i < PP) cfma(acc1[k], __ldg(U1 + i), __ldg(Fs + i));
           }
         }
-        a++;
-        b++;
-      } else if (sa < sb) {
-        const C* U0 = ptab + (int64_t)P.m2l_tab[a] * PP;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-          const int i = threadIdx.x + k * NT;
-          if (i < PP) cfma(acc0[k], __ldg(U0 + i), __ldg(Fs + i));
-        }
-        a++;
-      } else {
-        const C* U1 = ptab + (int64_t)P.m2l_tab[b] * PP;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-          const int i = threadIdx.x + k * NT;
-          if (i < PP) cfma(acc1[k], __ldg(U1 + i), __ldg(Fs + i));
-        }
-        b++;
       }
-    }
-    m2l_f2l<T, L, NT>(acc0, Js, Cb, D, Lx + t * LL);
-    if (two) m2l_f2l<T, L, NT>(acc1, Js, Cb, D, Lx + (t + 1) * LL);
+    };
+    if (ae <= Q::kCap && be <= Q::kCap)
+      merge([&](int jj, int x) { return qs.e[ph][jj][x]; });
+    else
+      merge([&](int jj, int x) { return x < Q::kCap ? qs.e[ph][jj][x] : q.direct(ph, jj, x); });
+    q.publish(ph ^ 1);
+    m2l_f2l<T, L, NT>(acc0, Js, Cb, D, Lx + t * LL, [&] { q.pointers(qs.item[ph ^ 1], u0 + 2 * qs.item[ph ^ 1], u1); },
+                      [&] { q.entries(); });
+    if (two) m2l_f2l<T, L, NT>(acc1, Js, Cb, D, Lx + t2 * LL, [] {}, [] {});
+    q.store(ph ^ 1);
+    __syncthreads();
   }
 }
 
@@ -1116,12 +1208,13 @@ __host__ __device__ constexpr bool m2l_rhs_joint() {
 }
 
 template <typename T, int L, int NT, int RB>
-__global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPlan P, int64_t t0, int64_t t1, int64_t f0, int64_t f1, int R,
+__global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1, int R,
                                                              const typename cpx_t<T>::type* __restrict__ F,
                                                              const typename cpx_t<T>::type* __restrict__ ptab,
                                                              typename cpx_t<T>::type* __restrict__ Lx,
                                                              unsigned long long* __restrict__ queue) {
   typedef typename cpx_t<T>::type C;
+  typedef M2LQueue<1, NT> Q;
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   constexpr bool JOINT = m2l_rhs_joint<T, L, RB>();
   constexpr int MS = JOINT ? RB : 1;  // inverse-DFT workspaces
@@ -1129,31 +1222,29 @@ __global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPl
   C* Js = reinterpret_cast<C*>(smem_raw);
   C* Cb = Js + MS * PP;
   C* D = Cb + MS * L * PD * PD;
-  __shared__ int64_t cur;
+  __shared__ typename Q::Shared qs;
   const int nb = R / RB;
-  const int64_t nwork = (t1 - t0) * nb;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
-    __syncthreads();
-    const int64_t w = cur;
-    if (w >= nwork) break;
-    const int64_t t = t0 + w / nb;
-    const int r0 = (int)(w % nb) * RB;
-    const int64_t eb = P.m2l_ptr[t], ee = P.m2l_ptr[t + 1];
+  const int64_t nwork = (u1 - u0) * nb;
+  Q q(qs, P, queue, nwork);
+  q.first(u0 + (int64_t)blockIdx.x / nb, u1);
+  __syncthreads();
+  for (int ph = 0; qs.item[ph] < nwork; ph ^= 1) {
+    q.fetch();
+    const int64_t w = qs.item[ph];
+    const int64_t t = P.m2l_tlist[u0 + w / nb];
+    const int r0 = (int)(w % nb) * RB, n = qs.len[ph][0];
     C acc[K][RB];
 #pragma unroll
     for (int k = 0; k < K; k++)
 #pragma unroll
       for (int b = 0; b < RB; b++) acc[k][b] = czero<C>();
-    for (int64_t e = eb; e < ee; e++) {
-      const int64_t src = P.m2l_src[e];
-      if (src < f0 || src >= f1) {  // entry outside this cone batch: a plan bug
+    auto add = [&](int2 e) {
+      if (e.x < f0 || e.x >= f1) {  // entry outside this cone batch: a plan bug
         if (threadIdx.x == 0) atomicExch(P.err, 1);
-        continue;
+        return;
       }
-      const C* Fs = F + ((src - f0) * R + r0) * PP;
-      const C* U = ptab + (int64_t)P.m2l_tab[e] * PP;
+      const C* Fs = F + ((e.x - f0) * R + r0) * PP;
+      const C* U = ptab + (int64_t)(uint32_t)e.y * PP;
 #pragma unroll
       for (int k = 0; k < K; k++) {
         const int i = threadIdx.x + k * NT;
@@ -1163,18 +1254,29 @@ __global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPl
           for (int b = 0; b < RB; b++) cfma(acc[k][b], u, __ldg(Fs + b * PP + i));
         }
       }
-    }
+    };
+    const int ns = min(n, Q::kCap);
+    for (int x = 0; x < ns; x++) add(qs.e[ph][0][x]);
+    for (int x = ns; x < n; x++) add(q.direct(ph, 0, x));
+    q.publish(ph ^ 1);
+    auto hook_a = [&] { q.pointers(qs.item[ph ^ 1], u0 + qs.item[ph ^ 1] / nb, u1); };
+    auto hook_b = [&] { q.entries(); };
     if constexpr (JOINT) {
-      m2l_f2l_rhs<T, L, NT, RB>(&acc[0][0], Js, Cb, D, Lx + (t * R + r0) * LL);
+      m2l_f2l_rhs<T, L, NT, RB>(&acc[0][0], Js, Cb, D, Lx + (t * R + r0) * LL, hook_a, hook_b);
     } else {
 #pragma unroll
       for (int b = 0; b < RB; b++) {
         C a[K];
 #pragma unroll
         for (int k = 0; k < K; k++) a[k] = acc[k][b];
-        m2l_f2l<T, L, NT>(a, Js, Cb, D, Lx + (t * R + r0 + b) * LL);
+        if (b == 0)
+          m2l_f2l<T, L, NT>(a, Js, Cb, D, Lx + (t * R + r0) * LL, hook_a, hook_b);
+        else
+          m2l_f2l<T, L, NT>(a, Js, Cb, D, Lx + (t * R + r0 + b) * LL, [] {}, [] {});
       }
     }
+    q.store(ph ^ 1);
+    __syncthreads();
   }
 }
 
@@ -2626,12 +2728,12 @@ struct Launch {
                                 (int)smem_m2l_rhs<(RB <= kMaxRB ? RB : 1)>());
   }
   template <int RB, int NT>
-  static void m2l_rhs_go(const DevPlan& dp, int64_t t0, int64_t t1, int64_t f0, int64_t f1, int R, const void* F,
+  static void m2l_rhs_go(const DevPlan& dp, int64_t u0, int64_t u1, int64_t f0, int64_t f1, int R, const void* F,
                          const void* ptab, void* Lx, unsigned long long* queue, int nsm, cudaStream_t s) {
     constexpr int RBE = RB <= kMaxRB ? RB : 1;
-    const int64_t nwork = (t1 - t0) * (R / RBE);
+    const int64_t nwork = (u1 - u0) * (R / RBE);
     const int grid = (int)std::min<int64_t>(nwork, (int64_t)nsm * m2l_rhs_ctas<T, NT, RBE>());
-    k_m2l_rhs<T, L, NT, RBE><<<grid, NT, smem_m2l_rhs<RBE>(), s>>>(dp, t0, t1, f0, f1, R, (const C*)F, (const C*)ptab,
+    k_m2l_rhs<T, L, NT, RBE><<<grid, NT, smem_m2l_rhs<RBE>(), s>>>(dp, u0, u1, f0, f1, R, (const C*)F, (const C*)ptab,
                                                           (C*)Lx, queue);
   }
   // the shared-memory-staged kernel: FP32, orders 3-6
@@ -2658,22 +2760,23 @@ struct Launch {
   }
   // M2L for R right-hand sides in blocks of rb (1, 2, 4 or 8; a divisor of
   // R, capped by the order's kMaxRB), or staged through shared memory
-  static void m2l_rhs(const DevPlan& dp, int64_t t0, int64_t t1, int64_t f0, int64_t f1, int R, int rb,
+  static void m2l_rhs(const DevPlan& dp, int64_t u0, int64_t u1, int64_t t0, int64_t t1, int64_t f0, int64_t f1,
+                      int R, int rb,
                       const void* F, const void* ptab, void* Lx, unsigned long long* queue, int nsm,
                       int64_t lgroup, cudaStream_t s) {
-    if (t1 <= t0) return;
+    if (u1 <= u0) return;
     cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
     if (m2l_bulk(dp, t0, t1, f0, f1, R, F, ptab, Lx, queue, nsm, lgroup, s)) return;
     if (rb > kMaxRB) rb = kMaxRB;
     while (rb > 1 && R % rb) rb >>= 1;
     if (rb >= 8)
-      m2l_rhs_go<8, 256>(dp, t0, t1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
+      m2l_rhs_go<8, 256>(dp, u0, u1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
     else if (rb >= 4)
-      m2l_rhs_go<4, 256>(dp, t0, t1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
+      m2l_rhs_go<4, 256>(dp, u0, u1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
     else if (rb >= 2)
-      m2l_rhs_go<2, 128>(dp, t0, t1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
+      m2l_rhs_go<2, 128>(dp, u0, u1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
     else
-      m2l_rhs_go<1, 128>(dp, t0, t1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
+      m2l_rhs_go<1, 128>(dp, u0, u1, f0, f1, R, F, ptab, Lx, queue, nsm, s);
   }
   static void p2m(const DevPlan& dp, const int32_t* leaves, int n, const void* q, const void* sig2, void* M, int R,
                   int d0, int d1, cudaStream_t s) {
@@ -2695,31 +2798,32 @@ struct Launch {
       k_l2l<T, L><<<grid_for(s1 - s0, NW), 32 * NW, 0, s>>>(dp, s0, s1, (const C*)sig, (const C*)sig2, (C*)Lc,
                                                                   (const C*)Lp, R, p0, p1);
   }
-  static void m2f(int64_t n, const void* M, void* F, cudaStream_t s) {
+  static void m2f(int64_t n, int R, const int32_t* slist, const void* M, void* F, cudaStream_t s) {
     constexpr int NW = M2FCfg<T, L>::NW;
-    if (n) k_m2f<T, L><<<grid_for(n, NW), 32 * NW, smem_m2f(), s>>>(n, (const C*)M, (C*)F);
+    if (n)
+      k_m2f<T, L><<<grid_for(n * R, NW), 32 * NW, smem_m2f(), s>>>(n * R, R, slist, (const C*)M, (C*)F);
   }
-  static void m2l(const DevPlan& dp, int64_t t0, int64_t t1, int64_t f0, int64_t f1, const void* F,
+  static void m2l(const DevPlan& dp, int64_t u0, int64_t u1, int64_t f0, int64_t f1, const void* F,
                   const void* ptab, void* Lx, unsigned long long* queue, int nsm, int nt, int pair,
                   cudaStream_t s) {
-    if (t1 <= t0) return;
+    if (u1 <= u0) return;
     cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
     if (nt != 128 && nt != 256) nt = NT;
     if (pair) {
-      const int grid = (int)std::min<int64_t>((t1 - t0 + 1) / 2, (int64_t)nsm * (2048 / nt));
+      const int grid = (int)std::min<int64_t>((u1 - u0 + 1) / 2, (int64_t)nsm * (2048 / nt));
       if (nt == 256)
-        k_m2l_pair<T, L, 256><<<grid, 256, smem_m2l(), s>>>(dp, t0, t1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx,
+        k_m2l_pair<T, L, 256><<<grid, 256, smem_m2l(), s>>>(dp, u0, u1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx,
                                                             queue);
       else
-        k_m2l_pair<T, L, 128><<<grid, 128, smem_m2l(), s>>>(dp, t0, t1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx,
+        k_m2l_pair<T, L, 128><<<grid, 128, smem_m2l(), s>>>(dp, u0, u1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx,
                                                             queue);
       return;
     }
-    const int grid = (int)std::min<int64_t>(t1 - t0, (int64_t)nsm * (2048 / nt));
+    const int grid = (int)std::min<int64_t>(u1 - u0, (int64_t)nsm * (2048 / nt));
     if (nt == 256)
-      k_m2l<T, L, 256><<<grid, 256, smem_m2l(), s>>>(dp, t0, t1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx, queue);
+      k_m2l<T, L, 256><<<grid, 256, smem_m2l(), s>>>(dp, u0, u1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx, queue);
     else
-      k_m2l<T, L, 128><<<grid, 128, smem_m2l(), s>>>(dp, t0, t1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx, queue);
+      k_m2l<T, L, 128><<<grid, 128, smem_m2l(), s>>>(dp, u0, u1, f0, f1, (const C*)F, (const C*)ptab, (C*)Lx, queue);
   }
   static void permute(int64_t n, const uint32_t* key, const uint16_t* perm, const void* tables, void* out,
                       cudaStream_t s) {

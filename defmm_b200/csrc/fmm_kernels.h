@@ -31,20 +31,24 @@ struct OpTable {
   // [p0, p1) (bases Lp)
   void (*l2l)(const DevPlan&, int64_t s0, int64_t s1, const void* sig, const void* sig2, void* Lc, const void* Lp,
               int R, int64_t p0, int64_t p1, cudaStream_t);
-  void (*m2f)(int64_t n, const void* M, void* F, cudaStream_t);
-  // M2L with the inverse DFT fused: adds into L of target slots [t0, t1)
+  // spectra of the n listed source slots (slist; R expansions each, M: base as
+  // above) into F: row i R + r for right-hand side r of the i-th
+  void (*m2f)(int64_t n, int R, const int32_t* slist, const void* M, void* F, cudaStream_t);
+  // M2L with the inverse DFT fused: adds into L of the listed target slots
+  // [u0, u1) (DevPlan::m2l_tlist) from the listed source slots [f0, f1) in F
   // nt: threads per CTA (128 or 256; 0 = the order's default); pair != 0:
   // two consecutive target slots per CTA sharing their common sources' loads
-  void (*m2l)(const DevPlan&, int64_t t0, int64_t t1, int64_t f0, int64_t f1, const void* F, const void* ptab,
+  void (*m2l)(const DevPlan&, int64_t u0, int64_t u1, int64_t f0, int64_t f1, const void* F, const void* ptab,
               void* Lx, unsigned long long* queue, int nsm, int nt, int pair, cudaStream_t);
   // The same for R right-hand sides (F: R spectra per source slot of the
   // batch, Lx: base as above), rb of them per CTA sharing each spectrum load.
   // lgroup > 0: the longest list total of kM2LGroup consecutive target
   // slots; the FP32 path at orders 3-6 then stages spectra through shared
   // memory with bulk copies, kM2LGroup target slots per CTA sharing each
-  // source's loads (bit-identical results); lgroup <= 0: one target slot per
-  // CTA.  F and ptab carry 16 bytes of slack after their last spectrum.
-  void (*m2l_rhs)(const DevPlan&, int64_t t0, int64_t t1, int64_t f0, int64_t f1, int R, int rb, const void* F,
+  // source's loads (bit-identical results; it takes all target slots
+  // [t0, t1) of the batch); lgroup <= 0: one target slot per CTA.  F and ptab carry 16 bytes of slack after their last spectrum.
+  void (*m2l_rhs)(const DevPlan&, int64_t u0, int64_t u1, int64_t t0, int64_t t1, int64_t f0, int64_t f1, int R,
+                  int rb, const void* F,
                   const void* ptab, void* Lx, unsigned long long* queue, int nsm, int64_t lgroup, cudaStream_t);
   // L2P of the leaves' slots with a direction in [d0, d1) into pfar (R per
   // particle), written (accum = false) or added

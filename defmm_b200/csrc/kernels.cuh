@@ -68,7 +68,11 @@ struct DevPlan {
   const int32_t *S_cslot, *S_cdir, *T_cslot, *T_cdir;
   // operators
   const int64_t *m2m_ptr, *l2l_ptr, *m2l_ptr;
-  const int32_t *m2m_child, *l2l_parent, *m2l_src;
+  const int32_t *m2m_child, *l2l_parent;
+  // M2L: per entry the source slot's position in m2l_slist and the permuted
+  // spectrum; target slots with a list and their pointers (one past the last)
+  const int32_t *m2l_src, *m2l_tlist, *m2l_slist;
+  const int64_t* m2l_cptr;
   const uint32_t* m2l_tab;
   const uint16_t* perm;
   const double* dirs;                          // all stages, 3 per direction

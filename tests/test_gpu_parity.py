@@ -470,3 +470,34 @@ def test_near_field_parts_and_block_widths(nrhs, gpu):
     for r in range(nrhs):
         assert rel(P[r], ex[r]) <= 1e-13
         assert rel(M[r], ex[r]) <= MIXED_TOL
+
+
+@pytest.mark.parametrize("order", [2, 3, 6])
+def test_m2l_long_and_empty_lists(order, gpu):
+    # M2L lists longer than what a CTA keeps in shared memory (64 entries),
+    # target slots without a list and source slots in none (both left out of
+    # the M2L and M2F), one and two target slots per CTA, 128 and 256 threads,
+    # and right-hand-side blocks over several direction groups
+    w = W.gaussian_blobs(6000, seed=4, wavelengths=3)
+    A = make(w.points, w.points, order, 16, w.kappa)
+    ptr, src, _ = A.m2l_entries()
+    n = np.diff(ptr)
+    assert n.max() > 128 and (n == 0).any() and len(np.unique(src)) < A.info("slots_S")
+    q = W.charges(w.n, 3)
+    ref = O.OracleFMM(w.points, w.points, order, 16, w.kappa, -1).gemv(q)
+    for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+        A.set_precision(prec)
+        first = A.matvec(q)
+        assert rel(first, ref) <= tol
+        for pair in (0, 1):
+            A.set_m2l_pairing(pair)
+            for nt in (128, 256):
+                A.set_launch(nt, 16)
+                assert np.array_equal(A.matvec(q), first)
+        A.set_blocking(5, 3)
+        P = A.matvec(np.stack([q, 2j * q, -q, q, q]))
+        assert rel(P[0], ref) <= tol and rel(P[1], 2j * ref) <= tol
+        A.set_blocking(16, 0)
+    # the lists dumped after the upload are the plan's
+    B = make(w.points, w.points, order, 16, w.kappa)
+    assert all(np.array_equal(a, b) for a, b in zip(A.m2l_entries(), B.m2l_entries()))

@@ -852,77 +852,23 @@ __device__ __forceinline__ void idft_line(const C (&v)[2 * L - 1], C (&out)[L]) 
   }
 }
 
-// Inverse DFT of one target slot's spectrum J (acc, K values per thread) into
-// its local expansion (fourier2geom, circulant.hpp:109-118):
+// Inverse DFTs of RB spectra of PP entries (acc[k RB + b]: the K values of
+// spectrum b, one per thread and k) into their local expansions at dst(b)
+// (fourier2geom, circulant.hpp:109-118):
 //   L_t[a,b,c] += (1/PP) sum_k J[k] conj(w)^(k0 a + k1 b + k2 c)
-// pruned to a,b,c < L, one line per thread per axis pass in shared memory.
-// Safe to call twice in a row: each pass reads only what the previous pass
-// wrote after the barrier between them.
-// a() and b() run after the first and the second barrier.
-template <typename T, int L, int NT, typename HookA, typename HookB>
-__device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, typename cpx_t<T>::type* Js,
-                                        typename cpx_t<T>::type* Cb, typename cpx_t<T>::type* D,
-                                        typename cpx_t<T>::type* __restrict__ Lt, HookA hook_a, HookB hook_b) {
+// pruned to a,b,c < L, one line per thread per axis pass, in place in Js (RB
+// PP entries of shared memory): a line's outputs go to entries that its own
+// thread has read.  One buffer instead of one per pass leaves the rest of
+// the SM's memory to L1, which serves part of the spectra.  Each axis pass
+// runs over the lines of all RB spectra, so the CTA's threads stay busy and
+// the transforms take three barriers together.  a() and b() run after the
+// first and the second one.  A barrier has to lie between this and the next
+// use of Js.
+template <typename T, int L, int NT, int RB, typename Dst, typename HookA, typename HookB>
+__device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, typename cpx_t<T>::type* Js, Dst dst,
+                                        HookA hook_a, HookB hook_b) {
   typedef typename cpx_t<T>::type C;
   constexpr int PD = 2 * L - 1, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
-  const T inv = T(1) / T(PP);
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    const int i = threadIdx.x + k * NT;
-    if (i < PP) Js[i] = acc[k];
-  }
-  __syncthreads();
-  hook_a();
-  for (int ln = threadIdx.x; ln < PD * PD; ln += NT) {  // axis 0: (k1,k2) lines -> a
-    C v[PD];
-#pragma unroll
-    for (int k0 = 0; k0 < PD; k0++) v[k0] = Js[k0 * PD * PD + ln];
-    C o[L];
-    idft_line<T, L>(v, o);
-#pragma unroll
-    for (int a = 0; a < L; a++) Cb[a * PD * PD + ln] = o[a];
-  }
-  __syncthreads();
-  hook_b();
-  for (int ln = threadIdx.x; ln < L * PD; ln += NT) {  // axis 1: (a,k2) lines -> b
-    const int a = ln / PD, k2 = ln % PD;
-    C v[PD];
-#pragma unroll
-    for (int k1 = 0; k1 < PD; k1++) v[k1] = Cb[(a * PD + k1) * PD + k2];
-    C o[L];
-    idft_line<T, L>(v, o);
-#pragma unroll
-    for (int b = 0; b < L; b++) D[(a * L + b) * PD + k2] = o[b];
-  }
-  __syncthreads();
-  for (int ln = threadIdx.x; ln < L * L; ln += NT) {  // axis 2: (a,b) lines -> c
-    C v[PD];
-#pragma unroll
-    for (int k2 = 0; k2 < PD; k2++) v[k2] = D[ln * PD + k2];
-    C s[L];
-    idft_line<T, L>(v, s);
-#pragma unroll
-    for (int c = 0; c < L; c++) {
-      C o = Lt[ln * L + c];
-      o.x += s[c].x * inv;
-      o.y += s[c].y * inv;
-      Lt[ln * L + c] = o;
-    }
-  }
-}
-
-// The same for the RB spectra of one target slot at once (acc[k RB + b]: the
-// K values of right-hand side b), their local expansions at Lt + b LL: each
-// axis pass runs over the lines of all RB spectra, so the CTA's threads stay
-// busy and the transform takes three barriers instead of 3 RB.  Every
-// output is computed by the operations of m2l_f2l for its spectrum.
-template <typename T, int L, int NT, int RB, typename HookA, typename HookB>
-__device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, typename cpx_t<T>::type* Js,
-                                            typename cpx_t<T>::type* Cb, typename cpx_t<T>::type* D,
-                                            typename cpx_t<T>::type* __restrict__ Lt, HookA hook_a, HookB hook_b) {
-  typedef typename cpx_t<T>::type C;
-  constexpr int PD = 2 * L - 1, PP = PD * PD * PD, K = (PP + NT - 1) / NT, LL = L * L * L;
-  constexpr int NB = L * PD * PD, ND = L * L * PD;  // per spectrum: Cb, D elements
   const T inv = T(1) / T(PP);
 #pragma unroll
   for (int k = 0; k < K; k++) {
@@ -934,48 +880,41 @@ __device__ __forceinline__ void m2l_f2l_rhs(const typename cpx_t<T>::type* acc, 
   __syncthreads();
   hook_a();
   for (int x = threadIdx.x; x < RB * PD * PD; x += NT) {  // axis 0: (k1,k2) lines -> a
-    const int b = x / (PD * PD), ln = x % (PD * PD);
-    const C* J = Js + b * PP;
-    C* Cq = Cb + b * NB;
-    C v[PD];
+    C* q = Js + x / (PD * PD) * PP + x % (PD * PD);
+    C v[PD], o[L];
 #pragma unroll
-    for (int k0 = 0; k0 < PD; k0++) v[k0] = J[k0 * PD * PD + ln];
-    C o[L];
+    for (int k = 0; k < PD; k++) v[k] = q[k * PD * PD];
     idft_line<T, L>(v, o);
 #pragma unroll
-    for (int a = 0; a < L; a++) Cq[a * PD * PD + ln] = o[a];
+    for (int a = 0; a < L; a++) q[a * PD * PD] = o[a];
   }
   __syncthreads();
   hook_b();
   for (int x = threadIdx.x; x < RB * L * PD; x += NT) {  // axis 1: (a,k2) lines -> b
-    const int r = x / (L * PD), ln = x % (L * PD);
-    const int a = ln / PD, k2 = ln % PD;
-    const C* Cq = Cb + r * NB;
-    C* Dq = D + r * ND;
-    C v[PD];
+    const int ln = x % (L * PD);
+    C* q = Js + x / (L * PD) * PP + ln / PD * (PD * PD) + ln % PD;
+    C v[PD], o[L];
 #pragma unroll
-    for (int k1 = 0; k1 < PD; k1++) v[k1] = Cq[(a * PD + k1) * PD + k2];
-    C o[L];
+    for (int k = 0; k < PD; k++) v[k] = q[k * PD];
     idft_line<T, L>(v, o);
 #pragma unroll
-    for (int b = 0; b < L; b++) Dq[(a * L + b) * PD + k2] = o[b];
+    for (int b = 0; b < L; b++) q[b * PD] = o[b];
   }
   __syncthreads();
   for (int x = threadIdx.x; x < RB * L * L; x += NT) {  // axis 2: (a,b) lines -> c
     const int r = x / (L * L), ln = x % (L * L);
-    const C* Dq = D + r * ND;
-    C* Lq = Lt + r * LL;
-    C v[PD];
+    const C* q = Js + r * PP + (ln / L * PD + ln % L) * PD;
+    C v[PD], s[L];
 #pragma unroll
-    for (int k2 = 0; k2 < PD; k2++) v[k2] = Dq[ln * PD + k2];
-    C s[L];
+    for (int k = 0; k < PD; k++) v[k] = q[k];
     idft_line<T, L>(v, s);
+    C* Lt = dst(r) + ln * L;
 #pragma unroll
     for (int c = 0; c < L; c++) {
-      C o = Lq[ln * L + c];
+      C o = Lt[c];
       o.x += s[c].x * inv;
       o.y += s[c].y * inv;
-      Lq[ln * L + c] = o;
+      Lt[c] = o;
     }
   }
 }
@@ -1061,8 +1000,6 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Js = reinterpret_cast<C*>(smem_raw);
-  C* Cb = Js + PP;
-  C* D = Cb + L * PD * PD;
   __shared__ typename Q::Shared qs;
   Q q(qs, P, queue, u1 - u0);
   q.first(u0 + (int64_t)blockIdx.x, u1);
@@ -1092,8 +1029,8 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(
     for (int x = 0; x < ns; x++) add(qs.e[ph][0][x]);
     for (int x = ns; x < n; x++) add(q.direct(ph, 0, x));
     q.publish(ph ^ 1);
-    m2l_f2l<T, L, NT>(acc, Js, Cb, D, Lx + t * LL, [&] { q.pointers(qs.item[ph ^ 1], u0 + qs.item[ph ^ 1], u1); },
-                      [&] { q.entries(); });
+    m2l_f2l<T, L, NT, 1>(acc, Js, [&](int) { return Lx + t * LL; }, [&] { q.pointers(qs.item[ph ^ 1], u0 + qs.item[ph ^ 1], u1); },
+                         [&] { q.entries(); });
     q.store(ph ^ 1);
     __syncthreads();
   }
@@ -1115,8 +1052,6 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Js = reinterpret_cast<C*>(smem_raw);
-  C* Cb = Js + PP;
-  C* D = Cb + L * PD * PD;
   __shared__ typename Q::Shared qs;
   const int64_t nwork = (u1 - u0 + 1) / 2;
   Q q(qs, P, queue, nwork);
@@ -1179,9 +1114,12 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_
     else
       merge([&](int jj, int x) { return x < Q::kCap ? qs.e[ph][jj][x] : q.direct(ph, jj, x); });
     q.publish(ph ^ 1);
-    m2l_f2l<T, L, NT>(acc0, Js, Cb, D, Lx + t * LL, [&] { q.pointers(qs.item[ph ^ 1], u0 + 2 * qs.item[ph ^ 1], u1); },
-                      [&] { q.entries(); });
-    if (two) m2l_f2l<T, L, NT>(acc1, Js, Cb, D, Lx + t2 * LL, [] {}, [] {});
+    m2l_f2l<T, L, NT, 1>(acc0, Js, [&](int) { return Lx + t * LL; }, [&] { q.pointers(qs.item[ph ^ 1], u0 + 2 * qs.item[ph ^ 1], u1); },
+                         [&] { q.entries(); });
+    if (two) {
+      __syncthreads();
+      m2l_f2l<T, L, NT, 1>(acc1, Js, [&](int) { return Lx + t2 * LL; }, [] {}, [] {});
+    }
     q.store(ph ^ 1);
     __syncthreads();
   }
@@ -1198,13 +1136,12 @@ template <typename T, int NT, int RB>
 constexpr int m2l_rhs_ctas() {
   return (sizeof(T) == 8 ? (RB >= 8 ? 512 : (RB >= 2 ? 768 : 1024)) : (RB >= 8 ? 768 : 1024)) / NT;
 }
-// FP32, orders <= 5, up to 4 right-hand sides per CTA: the inverse DFTs of
-// a target slot's RB spectra run together (m2l_f2l_rhs, RB workspaces in
-// shared memory, 43.5 KB at order 5, so 4 CTAs per SM still fit);
-// otherwise one after another
+// up to 4 right-hand sides per CTA whose spectra take at most 24 KB (FP32 at
+// orders <= 5, FP64 <= 4): the inverse DFTs of a target slot's RB spectra run
+// together; otherwise one after another
 template <typename T, int L, int RB>
 __host__ __device__ constexpr bool m2l_rhs_joint() {
-  return sizeof(T) == 4 && L <= 5 && RB > 1 && RB <= 4;
+  return RB > 1 && RB <= 4 && RB * (2 * L - 1) * (2 * L - 1) * (2 * L - 1) * 2 * sizeof(T) <= 24 * 1024;
 }
 
 template <typename T, int L, int NT, int RB>
@@ -1217,11 +1154,8 @@ __global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPl
   typedef M2LQueue<1, NT> Q;
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   constexpr bool JOINT = m2l_rhs_joint<T, L, RB>();
-  constexpr int MS = JOINT ? RB : 1;  // inverse-DFT workspaces
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Js = reinterpret_cast<C*>(smem_raw);
-  C* Cb = Js + MS * PP;
-  C* D = Cb + MS * L * PD * PD;
   __shared__ typename Q::Shared qs;
   const int nb = R / RB;
   const int64_t nwork = (u1 - u0) * nb;
@@ -1262,17 +1196,20 @@ __global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPl
     auto hook_a = [&] { q.pointers(qs.item[ph ^ 1], u0 + qs.item[ph ^ 1] / nb, u1); };
     auto hook_b = [&] { q.entries(); };
     if constexpr (JOINT) {
-      m2l_f2l_rhs<T, L, NT, RB>(&acc[0][0], Js, Cb, D, Lx + (t * R + r0) * LL, hook_a, hook_b);
+      m2l_f2l<T, L, NT, RB>(&acc[0][0], Js, [&](int r) { return Lx + (t * R + r0 + r) * LL; }, hook_a, hook_b);
     } else {
 #pragma unroll
       for (int b = 0; b < RB; b++) {
         C a[K];
 #pragma unroll
         for (int k = 0; k < K; k++) a[k] = acc[k][b];
-        if (b == 0)
-          m2l_f2l<T, L, NT>(a, Js, Cb, D, Lx + (t * R + r0) * LL, hook_a, hook_b);
-        else
-          m2l_f2l<T, L, NT>(a, Js, Cb, D, Lx + (t * R + r0 + b) * LL, [] {}, [] {});
+        auto dst = [&](int) { return Lx + (t * R + r0 + b) * LL; };
+        if (b == 0) {
+          m2l_f2l<T, L, NT, 1>(a, Js, dst, hook_a, hook_b);
+        } else {
+          __syncthreads();
+          m2l_f2l<T, L, NT, 1>(a, Js, dst, [] {}, [] {});
+        }
       }
     }
     q.store(ph ^ 1);
@@ -2692,7 +2629,7 @@ struct Launch {
   static constexpr int P = 2 * L - 1, LL = L * L * L, PP = P * P * P;
   static constexpr int NT = PP > 1024 ? 256 : 128;
   static size_t smem_m2f() { return sizeof(C) * M2FCfg<T, L>::PER_WARP * M2FCfg<T, L>::NW; }
-  static size_t smem_m2l() { return sizeof(C) * (PP + L * P * P + L * L * P); }
+  static size_t smem_m2l() { return sizeof(C) * PP; }
   template <int RB>
   static size_t smem_m2l_rhs() { return (m2l_rhs_joint<T, L, RB>() ? RB : 1) * smem_m2l(); }
   static cudaError_t setup(const double* mats) {

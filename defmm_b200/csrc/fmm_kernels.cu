@@ -98,9 +98,12 @@ __global__ void k_scatter(const double2* __restrict__ pnear, const double2* __re
 // points: Z[j][l] is built once per chunk in shared memory (point-major, l
 // padded to LLP = 32 R); each warp takes S of the leaf's slots at a time,
 // writes their W column block, and every lane accumulates an R x S register
-// tile (expansion entries R lane .. R lane + R - 1, all S slots) over the
-// chunk's points: per point one R-wide load of Z and S broadcast loads of W
-// feed 2 R S FMAs.
+// tile (expansion entries lane + 32 e, all S slots, so signatures and results
+// are read and written at unit stride) over the chunk's points: per point R
+// loads of Z and S broadcast loads of W feed 2 R S FMAs.  Latency bounds it
+// (the signatures' loads), so a chunk is small enough for 4 CTAs per SM:
+// sphere 250k FP64 5.7 -> 4.0 ms against entries R lane .. R lane + R - 1 and
+// chunks of 64 points, spheroid 500k mixed order 6 9.1 -> 5.5 ms.
 template <typename T, int L>
 struct P2MCfg {
   static constexpr int LL = L * L * L;
@@ -108,7 +111,7 @@ struct P2MCfg {
   static constexpr int LLP = 32 * R;
   static constexpr int S0 = (sizeof(T) == 4 ? 32 : 16) / R;
   static constexpr int S = S0 < 1 ? 1 : (S0 > (sizeof(T) == 4 ? 8 : 4) ? (sizeof(T) == 4 ? 8 : 4) : S0);
-  static constexpr int NPB0 = 65536 / (LLP * (int)sizeof(T));
+  static constexpr int NPB0 = 40960 / (LLP * (int)sizeof(T));
   static constexpr int NPB = NPB0 > 64 ? 64 : NPB0;  // points per chunk
   typedef typename cpx_t<T>::type C;
   // shared memory: Z, point offsets, basis values, W blocks of 4 warps,
@@ -166,12 +169,12 @@ __device__ __forceinline__ void p2m_group(const DevPlan& P, int64_t j0, int ns, 
     for (int e = 0; e < RE; e++)
 #pragma unroll
       for (int s = 0; s < SS; s++) acc[e][s] = czero<C>();
-    const T* zl = Zs + lane * RE;
+    const T* zl = Zs + lane;
     for (int j = 0; j < np; j++) {
       T z[RE];
       C w[SS];
 #pragma unroll
-      for (int e = 0; e < RE; e++) z[e] = zl[j * LLP + e];
+      for (int e = 0; e < RE; e++) z[e] = zl[j * LLP + 32 * e];
 #pragma unroll
       for (int s = 0; s < SS; s++) w[s] = Ws[j * SS + s];
 #pragma unroll
@@ -185,7 +188,7 @@ __device__ __forceinline__ void p2m_group(const DevPlan& P, int64_t j0, int ns, 
         const int slot = P.S_cslot[j0 + s], d = P.S_cdir[j0 + s];
 #pragma unroll
         for (int e = 0; e < RE; e++) {
-          const int l = lane * RE + e;
+          const int l = lane + 32 * e;
           if (l < LL) {
             const C a = hf ? cmulc(s2[(int64_t)d * LL + l], acc[e][s]) : acc[e][s];
             C* out = M + ((int64_t)slot * R + r) * LL + l;
@@ -206,12 +209,15 @@ __device__ __forceinline__ void p2m_group(const DevPlan& P, int64_t j0, int ns, 
 
 // M: base of the expansions written here (slot s, right-hand side r at
 // M + (s R + r) LL); q: tree-order charges, R per particle (q[j R + r]);
-// only the leaf slots with a direction in [d0, d1) are computed.
+// only the leaf slots with a direction in [d0, d1) are computed.  A leaf's
+// slots are shared by `split` CTAs (each builds Z for itself) where there are
+// too few leaves to fill the chip.
 template <typename T, int L>
 __global__ void __launch_bounds__(128) k_p2m(DevPlan P, const int32_t* __restrict__ leaves, int nleaves,
                                              const typename cpx_t<T>::type* __restrict__ q,
                                              const typename cpx_t<T>::type* __restrict__ sig2,
-                                             typename cpx_t<T>::type* __restrict__ M, int R, int d0, int d1) {
+                                             typename cpx_t<T>::type* __restrict__ M, int R, int d0, int d1,
+                                             int split) {
   typedef typename cpx_t<T>::type C;
   typedef P2MCfg<T, L> G;
   constexpr int LL = G::LL, LLP = G::LLP, NPB = G::NPB, S = G::S;
@@ -225,8 +231,8 @@ __global__ void __launch_bounds__(128) k_p2m(DevPlan P, const int32_t* __restric
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   C* Ws = Wall + warp * NPB * S;
   C* Es = Eall + warp * NPB * S;
-  for (int li = blockIdx.x; li < nleaves; li += gridDim.x) {
-    const int c = leaves[li];
+  for (int64_t w = blockIdx.x; w < (int64_t)nleaves * split; w += gridDim.x) {
+    const int c = leaves[w / split], part = (int)(w % split);
     const int n = P.S_nprt[c], f = P.S_first[c];
     const double4 ct = P.S_ctr[c];
     const int lv = P.S_lvl[c];
@@ -235,7 +241,7 @@ __global__ void __launch_bounds__(128) k_p2m(DevPlan P, const int32_t* __restric
     int64_t sb, se;
     dir_range(P.S_cptr, P.S_cdir, c, d0, d1, &sb, &se);
     const int nslots = (int)(se - sb);
-    if (nslots == 0) continue;
+    if (nslots <= 4 * S * part) continue;
     const double* dirs = P.dirs + P.dir_off[h] * 3;
     const C* s2 = sig2 + P.sig_off[h];
     for (int p0 = 0; p0 < n; p0 += NPB) {
@@ -262,7 +268,7 @@ __global__ void __launch_bounds__(128) k_p2m(DevPlan P, const int32_t* __restric
         Zs[o] = z;
       }
       __syncthreads();
-      for (int g0 = warp * S; g0 < nslots; g0 += 4 * S) {
+      for (int g0 = (4 * part + warp) * S; g0 < nslots; g0 += 4 * S * split) {
         const int ns = min(S, nslots - g0);
         if (ns == 1)
           p2m_group<T, L, 1>(P, sb + g0, 1, hf, p0 == 0, np, Zs, yc, qs, Ws, Es, dirs, s2, M, R, lane);
@@ -2717,9 +2723,13 @@ struct Launch {
   }
   static void p2m(const DevPlan& dp, const int32_t* leaves, int n, const void* q, const void* sig2, void* M, int R,
                   int d0, int d1, cudaStream_t s) {
-    if (n)
-      k_p2m<T, L><<<grid_for(n, 1), 128, P2MCfg<T, L>::smem(R), s>>>(dp, leaves, n, (const C*)q, (const C*)sig2,
-                                                                     (C*)M, R, d0, d1);
+    if (!n) return;
+    // parts until there are 16 CTAs per SM (4 are resident): the three P2M
+    // launches (95, 364 and 938 leaves) of blobs of 15,001 points, order 4,
+    // three right-hand sides, FP64 took 134 us whole and take 95 us in parts
+    const int split = std::max(1, std::min(4, 148 * 16 / n));
+    k_p2m<T, L><<<grid_for((int64_t)n * split, 1), 128, P2MCfg<T, L>::smem(R), s>>>(
+        dp, leaves, n, (const C*)q, (const C*)sig2, (C*)M, R, d0, d1, split);
   }
   static void m2m(const DevPlan& dp, int64_t s0, int64_t s1, const void* sig, const void* sig2, void* Mp,
                   const void* Mc, int R, cudaStream_t s) {

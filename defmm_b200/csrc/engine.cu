@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/defmm_b200.h"
+#include "device_slab.hpp"
 #include "engine_internal.h"
 #include "fmm_kernels.h"
 #include "m2l_lists.hpp"
@@ -67,7 +68,8 @@ struct defmm_handle {
   int device = -1;
   cudaStream_t st = nullptr, st2 = nullptr;  // own stream; near field
   cudaStream_t cur = nullptr;                // stream of the gemv in progress (phase events)
-  std::vector<void*> plan_allocs;  // freed when the plan is rebuilt
+  std::vector<void*> plan_allocs;  // freed when the plan is rebuilt, like the slab's arrays
+  dfb::DeviceSlab plan_slab;
   DevPlan dp;
   const dfb::OpTable* ops = nullptr;
   int ops_prec = -1;
@@ -204,15 +206,12 @@ template <typename V>
 int upload(defmm_handle* h, const std::vector<V>& v, const V** out) {
   *out = nullptr;
   if (v.empty()) return 0;
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, v.size() * sizeof(V));
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return h->fail(DEFMM_ERR_MEMORY, std::string("device allocation failed: ") + cudaGetErrorString(e));
-  }
-  h->plan_allocs.push_back(p);
+  void* p = h->plan_slab.get(v.size() * sizeof(V));
+  if (!p)
+    return h->fail(DEFMM_ERR_MEMORY,
+                   std::string("device allocation failed: ") + cudaGetErrorString(cudaErrorMemoryAllocation));
   h->dev_bytes += v.size() * sizeof(V);
-  e = cudaMemcpy(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice);
+  const cudaError_t e = cudaMemcpy(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return h->fail(DEFMM_ERR_CUDA, cudaGetErrorString(e));
   *out = static_cast<const V*>(p);
   return 0;
@@ -241,6 +240,7 @@ void free_plan_device(defmm_handle* h) {
   drop_graph(h);
   for (void* p : h->plan_allocs) cudaFree(p);
   h->plan_allocs.clear();
+  h->plan_slab.release();
   free_buf(h->M);
   free_buf(h->Lx);
   free_buf(h->F);
@@ -482,9 +482,8 @@ int upload_plan(defmm_handle* h) {
   {  // target slots with a list, source slots in some list; entries renumbered
      // to the latter (last: an upload that failed before can be repeated)
     const size_t nT1 = (size_t)p.sT.n + 1, bytes = nT1 * 8 + nT1 * 4 + (size_t)(p.sS.n + 1) * 4;
-    void* cp = nullptr;
-    CK(cudaMalloc(&cp, bytes));
-    h->plan_allocs.push_back(cp);
+    void* cp = h->plan_slab.get(bytes);
+    if (!cp) return h->fail(DEFMM_ERR_MEMORY, "M2L lists: out of device memory");
     h->dev_bytes += bytes;
     int64_t* cptr = static_cast<int64_t*>(cp);
     int32_t* tl = reinterpret_cast<int32_t*>(cptr + nT1);
@@ -497,7 +496,7 @@ int upload_plan(defmm_handle* h) {
     std::string e;
     const int64_t nent = p.m2l_ptr.empty() ? 0 : p.m2l_ptr.back();
     st = dfb::device_m2l_lists(d.m2l_ptr, const_cast<int32_t*>(d.m2l_src), nent, p.sT.n, p.sS.n, atT, atS, cptr, tl,
-                               sl, e);
+                               sl, h->plan_slab, e);
     if (st) return h->fail(st == -5 ? DEFMM_ERR_MEMORY : DEFMM_ERR_CUDA, e);
     h->m2l_ranked = true;
     d.m2l_cptr = cptr;
@@ -1676,13 +1675,8 @@ int defmm_prcmpt(defmm_handle* h, int L, int Ncrit, double kappa, int lvMAX) {
                            (int64_t)h->trg.size() / 3, L, Ncrit, kappa, lvMAX, e, walker, sorter.get());
   // arrays the walk left on the device belong to this handle's plan (also
   // when the build failed part way)
-  for (void* q : {h->plan.dev_m2l_src, h->plan.dev_m2l_tab, h->plan.dev_m2m_ptr, h->plan.dev_m2m_child,
-                  h->plan.dev_l2l_ptr, h->plan.dev_l2l_parent, h->plan.dev_cslot_T, h->plan.dev_cdir_T,
-                  h->plan.dev_cslot_S, h->plan.dev_cdir_S, h->plan.dev_scell_T, h->plan.dev_sdir_T,
-                  h->plan.dev_scell_S, h->plan.dev_sdir_S})
-    if (q) h->plan_allocs.push_back(q);
-  h->plan_allocs.insert(h->plan_allocs.end(), h->plan.dev_near_allocs.begin(), h->plan.dev_near_allocs.end());
-  h->plan.dev_near_allocs.clear();
+  h->plan_allocs.insert(h->plan_allocs.end(), h->plan.dev_allocs.begin(), h->plan.dev_allocs.end());
+  h->plan.dev_allocs.clear();
   if (st) return h->fail(st == -4 ? DEFMM_ERR_CUDA : st == -5 ? DEFMM_ERR_MEMORY : st, e);
   h->walked_on_device = walker != nullptr;
   if (h->plan.lv.nlvl > 32) return h->fail(DEFMM_ERR_DEPTH, "more than 32 tree levels");

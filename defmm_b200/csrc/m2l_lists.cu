@@ -59,14 +59,14 @@ unsigned blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 
 int device_m2l_lists(const int64_t* ptr, int32_t* src, int64_t nent, int64_t nT, int64_t nS,
                      std::vector<int64_t>& atT, std::vector<int64_t>& atS, int64_t* cptr, int32_t* tlist,
-                     int32_t* slist, std::string& err) {
+                     int32_t* slist, DeviceSlab& slab, std::string& err) {
   const int64_t nmax = std::max(nT, nS) + 1, na = (int64_t)std::max(atT.size(), atS.size());
   size_t scan = 0;
   char* tmp = nullptr;
   cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, scan, (int32_t*)nullptr, (int32_t*)nullptr, nmax);
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t flag_b = up(nmax * 4), at_b = up(na * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, 2 * flag_b + 2 * at_b + scan);
+  if (e == cudaSuccess && !(tmp = (char*)slab.get(2 * flag_b + 2 * at_b + scan))) e = cudaErrorMemoryAllocation;
   int32_t *flag = (int32_t*)tmp, *rank = (int32_t*)(tmp + flag_b);
   int64_t *at = (int64_t*)(tmp + 2 * flag_b), *got = (int64_t*)(tmp + 2 * flag_b + at_b);
   void* cubtmp = tmp + 2 * flag_b + 2 * at_b;
@@ -94,7 +94,7 @@ int device_m2l_lists(const int64_t* ptr, int32_t* src, int64_t nent, int64_t nT,
   }
   const cudaError_t d = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = d;
-  if (tmp) cudaFree(tmp);
+  if (tmp) slab.drop(tmp);
   if (e == cudaSuccess) return 0;
   cudaGetLastError();
   err = std::string("M2L list compaction: ") + cudaGetErrorString(e);

@@ -26,6 +26,7 @@
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
 
+#include "device_slab.hpp"
 #include "plan.hpp"
 #include "plan_device.hpp"
 
@@ -346,42 +347,20 @@ __global__ void k_split_fill(int64_t nch, const int64_t* __restrict__ ptr, const
 // Device memory of one build: scratch freed at the end, outputs handed to
 // the plan on success (freed here on failure).
 struct Mem {
-  std::vector<void*> tmp, out;
+  DeviceSlab tmp, out;
   void* cub = nullptr;
   size_t cub_bytes = 0;
-  ~Mem() {
-    for (void* q : tmp) cudaFree(q);
-    for (void* q : out) cudaFree(q);
-    if (cub) cudaFree(cub);
-  }
   template <class T>
   T* get(int64_t n, bool keep = false) {
-    void* q = nullptr;
-    if (cudaMalloc(&q, (size_t)std::max<int64_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    (keep ? out : tmp).push_back(q);
-    return static_cast<T*>(q);
+    return static_cast<T*>((keep ? out : tmp).get((size_t)std::max<int64_t>(n, 1) * sizeof(T)));
   }
-  void drop(void* q) {
-    for (auto& x : tmp)
-      if (x == q) {
-        cudaFree(q);
-        x = nullptr;
-      }
-  }
+  void drop(void* q) { tmp.drop(q); }
   bool temp(size_t need) {
     if (need <= cub_bytes) return true;
-    if (cub) cudaFree(cub);
-    cub = nullptr;
-    cub_bytes = 0;
-    if (cudaMalloc(&cub, need) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    cub_bytes = need;
-    return true;
+    if (cub) tmp.drop(cub);
+    cub = tmp.get(need);
+    cub_bytes = cub ? need : 0;
+    return cub != nullptr;
   }
 };
 
@@ -719,8 +698,8 @@ int device_near_lists(Plan& p, const int2* d_near, int64_t npair, std::string& e
   o.p2p_order = it.order;
   NL_CK(cudaDeviceSynchronize());
   o.on = true;
-  p.dev_near_allocs.insert(p.dev_near_allocs.end(), M.out.begin(), M.out.end());
-  M.out.clear();
+  const std::vector<void*> kept = M.out.take();
+  p.dev_allocs.insert(p.dev_allocs.end(), kept.begin(), kept.end());
   return 0;
 }
 

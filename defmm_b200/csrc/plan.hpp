@@ -163,8 +163,7 @@ struct Plan {
   int64_t sym_scratch = 0;                   // scratch slots (one complex each)
   // The same near-field lists built on the device by the device walk (the
   // host vectors p2p_*, self_*, sym_*, red_* above then stay empty): device
-  // arrays with the host build's contents, and their sizes.  The operator
-  // that owns the plan releases them (dev_near_allocs).
+  // arrays with the host build's contents, and their sizes.
   struct NearOnDevice {
     bool on = false;
     int64_t nchunk = 0, p2p_items = 0, n_self_order = 0, sym_items = 0, n_red = 0;
@@ -178,7 +177,9 @@ struct Plan {
     const int32_t *red_first = nullptr, *red_n = nullptr;
     const int64_t *red_ptr = nullptr, *red_off = nullptr;
   } nd;
-  std::vector<void*> dev_near_allocs;
+  // the device allocations behind every dev_* array and nd above (pieces of
+  // them): the operator that owns the plan frees them
+  std::vector<void*> dev_allocs;
   // sizes of the near-field lists wherever they were built
   int64_t near_chunks() const { return nd.on ? nd.nchunk : (int64_t)p2p_tfirst.size(); }
   int64_t near_items() const { return nd.on ? nd.p2p_items : (int64_t)p2p_order.size(); }

@@ -13,6 +13,7 @@
 #include <memory>
 #include <cstring>
 
+#include "device_slab.hpp"
 #include "fp64_math.hpp"
 #include "plan.hpp"
 #include "plan_device.hpp"
@@ -362,23 +363,26 @@ inline unsigned nblk(int64_t n, int b = 256) { return (unsigned)std::max<int64_t
 
 // Device buffers of one walk; everything is freed at the end.
 struct Arena {
-  std::vector<void*> all;
-  ~Arena() {
-    for (void* p : all) cudaFree(p);
+  DeviceSlab slab;
+  template <typename T>
+  T* get(size_t n) {
+    return static_cast<T*>(slab.get(std::max<size_t>(1, n) * sizeof(T)));
+  }
+  void drop(void* p) { slab.drop(p); }
+};
+
+// Device arrays that stay with the plan, whatever comes of the walk.
+struct Keep {
+  Plan& p;
+  DeviceSlab slab;
+  explicit Keep(Plan& plan) : p(plan) {}
+  ~Keep() {
+    const std::vector<void*> v = slab.take();
+    p.dev_allocs.insert(p.dev_allocs.end(), v.begin(), v.end());
   }
   template <typename T>
   T* get(size_t n) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(T)) != cudaSuccess) return nullptr;
-    all.push_back(p);
-    return static_cast<T*>(p);
-  }
-  void drop(void* p) {
-    auto it = std::find(all.begin(), all.end(), p);
-    if (it != all.end()) {
-      cudaFree(p);
-      all.erase(it);
-    }
+    return static_cast<T*>(slab.get(std::max<size_t>(1, n) * sizeof(T)));
   }
 };
 
@@ -411,7 +415,6 @@ struct DeviceWalker final : LevelWalker {
   do {                                                           \
     ptr = A.get<T>(n);                                           \
     if (!ptr) {                                                  \
-      cudaGetLastError();                                        \
       err = "device plan: out of device memory";                 \
       return -5;                                                 \
     }                                                            \
@@ -430,6 +433,7 @@ int DeviceWalker::walk(Plan& p, LevelWalk& walk, std::string& err) {
   const Levels& v = p.lv;
   const int nlvl = v.nlvl;
   Arena A;
+  Keep K(p);
   // cells per level (DFS order) and level-local indices, as the host walk
   std::vector<std::vector<int32_t>> lcT(nlvl), lcS(nlvl);
   std::vector<int32_t> locT(p.T.ncell), locS(p.S.ncell);
@@ -786,9 +790,7 @@ int DeviceWalker::walk(Plan& p, LevelWalk& walk, std::string& err) {
       DW_ALLOC(cnt, int32_t, nc + 1);
       DW_ALLOC(ptr, int64_t, nc + 1);
       for (void** q : {dcell, ddirs, dslot, ddir})
-        if (cudaMalloc(q, std::max<int64_t>(1, n) * sizeof(int32_t)) != cudaSuccess) {  // handed to the plan's owner
-          cudaGetLastError();
-          *q = nullptr;
+        if (!(*q = K.get<int32_t>(n))) {
           err = "device plan: out of device memory";
           return -5;
         }
@@ -848,20 +850,18 @@ int DeviceWalker::walk(Plan& p, LevelWalk& walk, std::string& err) {
     int64_t* cnt;  // 64-bit, so that the scan's sums cannot overflow
     DW_ALLOC(cnt, int64_t, n + 1);
     DW_CK(cudaMemset(cnt, 0, (n + 1) * sizeof(int64_t)));
-    int64_t* ptr = nullptr;
-    if (cudaMalloc(&ptr, (n + 1) * sizeof(int64_t)) != cudaSuccess) {
-      cudaGetLastError();
+    int64_t* ptr = K.get<int64_t>(n + 1);
+    if (!ptr) {
       err = "device plan: out of device memory";
       return -5;
     }
-    *ptr_out = ptr;  // handed to the plan's owner (also on error: freed there)
+    *ptr_out = ptr;
     for (int pass = 0; pass < 2; pass++) {
       if (pass == 1) {
         int s2 = scan(cnt, ptr, n + 1);
         if (s2) return s2;
         if ((s2 = last(ptr, n, *n_out))) return s2;
-        if (cudaMalloc(ent_out, std::max<int64_t>(1, *n_out) * sizeof(int32_t)) != cudaSuccess) {
-          cudaGetLastError();
+        if (!(*ent_out = K.get<int32_t>(*n_out))) {
           err = "device plan: out of device memory";
           return -5;
         }
@@ -1020,42 +1020,34 @@ int DeviceWalker::walk(Plan& p, LevelWalk& walk, std::string& err) {
   DW_ALLOC(pid, int32_t, ntab + 1);
   DW_CK(cudaMemset(cnt, 0, (nslot + 1) * sizeof(int32_t)));
   DW_CK(cudaMemset(used, 0, (ntab + 1) * sizeof(int32_t)));
-  void *src_out = nullptr, *key_out = nullptr;  // handed to the plan's owner
-  DW_CK(cudaMalloc(&src_out, std::max<int64_t>(1, n) * sizeof(int32_t)));
-  if (cudaMalloc(&key_out, std::max<int64_t>(1, n) * sizeof(uint32_t)) != cudaSuccess) {
-    cudaFree(src_out);
-    cudaGetLastError();
+  void *src_out = K.get<int32_t>(n), *key_out = K.get<uint32_t>(n);
+  if (!src_out || !key_out) {
     err = "device plan: out of device memory";
     return -5;
   }
-  auto fail_out = [&](int code) {
-    cudaFree(src_out);
-    cudaFree(key_out);
-    return code;
-  };
   if (n) {
     k_count<<<nblk(n), 256>>>(n, all_ts, cnt);
     k_gather_entries<<<nblk(n), 256>>>(n, idx_out, all_ss, all_tab, (int32_t*)src_out, (uint32_t*)key_out, used);
   }
-  if (cudaGetLastError() != cudaSuccess) return fail_out(-4);
+  if (cudaGetLastError() != cudaSuccess) return -4;
   int32_t* pos = nullptr;
   pos = A.get<int32_t>(nslot + 1);
-  if (!pos) return fail_out(-5);
-  if ((st = scan(cnt, pos, nslot + 1)) || (st = scan(used, pid, ntab + 1))) return fail_out(st);
+  if (!pos) return -5;
+  if ((st = scan(cnt, pos, nslot + 1)) || (st = scan(used, pid, ntab + 1))) return st;
   if (n) k_renumber<<<nblk(n), 256>>>(n, pid, (uint32_t*)key_out);
   const cudaError_t esync = cudaDeviceSynchronize();
   p.step("walk: far entries by target slot (radix sorts)", tstep);
   if (esync != cudaSuccess) {
     cudaGetLastError();
     err = "device plan: M2L grouping failed";
-    return fail_out(-4);
+    return -4;
   }
   std::vector<int32_t> ph(nslot + 1), uh(ntab);
   if (cudaMemcpy(ph.data(), pos, (nslot + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess ||
       (ntab && cudaMemcpy(uh.data(), used, ntab * sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess)) {
     cudaGetLastError();
     err = "device plan: copy of the M2L grouping failed";
-    return fail_out(-4);
+    return -4;
   }
   p.m2l_ptr.assign(ph.begin(), ph.end());
   p.ptab_key.clear();
@@ -1127,10 +1119,15 @@ struct DeviceSorter final : TreeSorter {
   void* tmp = nullptr;
   size_t tmp_bytes = 0;
   cudaStream_t st = nullptr;
+  DeviceSlab slab;
+  template <typename P>
+  cudaError_t take(P** q, size_t bytes) {
+    *q = static_cast<P*>(slab.get(bytes));
+    return *q ? cudaSuccess : cudaErrorMemoryAllocation;
+  }
   void release() {
-    for (void* p : {(void*)pts, (void*)order, (void*)order2, (void*)cf, (void*)key, (void*)at, (void*)cnt,
-                    (void*)code, (void*)first, (void*)childf, (void*)ctr, (void*)split, tmp})
-      if (p) cudaFree(p);
+    if (st) cudaStreamSynchronize(st);
+    slab.release();
     pts = nullptr;
     order = order2 = cf = key = at = cnt = nullptr;
     code = nullptr;
@@ -1157,11 +1154,10 @@ struct DeviceSorter final : TreeSorter {
     while (bits < 31 && ((int64_t)1 << bits) <= n) bits++;
     cudaError_t e;
     if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaMalloc(&pts, 24 * (size_t)n)) != cudaSuccess ||
-        (e = cudaMalloc(&order, 4 * (size_t)n)) != cudaSuccess ||
-        (e = cudaMalloc(&order2, 4 * (size_t)n)) != cudaSuccess || (e = cudaMalloc(&cf, 4 * (size_t)n)) != cudaSuccess ||
-        (e = cudaMalloc(&key, 4 * (size_t)n)) != cudaSuccess || (e = cudaMalloc(&at, 4 * (size_t)n)) != cudaSuccess ||
-        (e = cudaMalloc(&code, (size_t)n)) != cudaSuccess)
+        (e = take(&pts, 24 * (size_t)n)) != cudaSuccess || (e = take(&order, 4 * (size_t)n)) != cudaSuccess ||
+        (e = take(&order2, 4 * (size_t)n)) != cudaSuccess || (e = take(&cf, 4 * (size_t)n)) != cudaSuccess ||
+        (e = take(&key, 4 * (size_t)n)) != cudaSuccess || (e = take(&at, 4 * (size_t)n)) != cudaSuccess ||
+        (e = take(&code, (size_t)n)) != cudaSuccess)
       return fail(err, "allocation", e);
     if ((e = cudaMemcpyAsync(pts, p, 24 * (size_t)n, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (e = cudaMemsetAsync(cf, 0, 4 * (size_t)n, st)) != cudaSuccess ||
@@ -1172,7 +1168,7 @@ struct DeviceSorter final : TreeSorter {
     if ((e = cub::DeviceRadixSort::SortPairs(nullptr, need, key, cf, order, order2, (int)n, 0, bits, st)) !=
         cudaSuccess)
       return fail(err, "sort size", e);
-    if ((e = cudaMalloc(&tmp, need)) != cudaSuccess) return fail(err, "allocation", e);
+    if ((e = take(&tmp, need)) != cudaSuccess) return fail(err, "allocation", e);
     tmp_bytes = need;
     return 0;
   }
@@ -1181,15 +1177,15 @@ struct DeviceSorter final : TreeSorter {
     cudaError_t e;
     if (m > cap) {
       for (void* q : {(void*)first, (void*)childf, (void*)ctr, (void*)split, (void*)cnt})
-        if (q) cudaFree(q);
+        if (q) slab.drop(q);
       first = childf = nullptr;
       ctr = nullptr;
       split = nullptr;
       cnt = nullptr;
       cap = std::max<int64_t>(m, 1024);
-      if ((e = cudaMalloc(&first, 8 * cap)) != cudaSuccess || (e = cudaMalloc(&childf, 64 * cap)) != cudaSuccess ||
-          (e = cudaMalloc(&ctr, 24 * cap)) != cudaSuccess || (e = cudaMalloc(&split, cap)) != cudaSuccess ||
-          (e = cudaMalloc(&cnt, 32 * cap)) != cudaSuccess)
+      if ((e = take(&first, 8 * cap)) != cudaSuccess || (e = take(&childf, 64 * cap)) != cudaSuccess ||
+          (e = take(&ctr, 24 * cap)) != cudaSuccess || (e = take(&split, cap)) != cudaSuccess ||
+          (e = take(&cnt, 32 * cap)) != cudaSuccess)
         return fail(err, "allocation", e);
     }
     if ((e = cudaMemcpyAsync(first, f, 8 * m, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
@@ -1327,16 +1323,12 @@ int device_plan_tables(const Plan& p, double2* tables, double2* sig, double2* si
     cudaGetLastError();
     return -4;
   };
-  std::vector<void*> tmp;
+  DeviceSlab tmp;
   auto up = [&](const void* src, size_t bytes, void** dst) -> cudaError_t {
-    cudaError_t e = cudaMalloc(dst, std::max<size_t>(1, bytes));
-    if (e != cudaSuccess) return e;
-    tmp.push_back(*dst);
+    if (!(*dst = tmp.get(bytes))) return cudaErrorMemoryAllocation;
     return bytes ? cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
   };
-  auto release = [&]() {
-    for (void* q : tmp) cudaFree(q);
-  };
+  auto release = [&]() { tmp.release(); };
   cudaError_t e = cudaSuccess;
   const int64_t ntab = (int64_t)p.tab_fund.size();
   if (ntab) {

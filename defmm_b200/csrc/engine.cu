@@ -844,7 +844,7 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
   rec(h, 2 * PH_TOTAL);
   if (!tuning) {
     dfb::launch_gather(fp64, qin, d.S_perm, h->q.p, nS, 0, 0, 1, s);
-    nl_ += 1 + (p.p2m_leaf.empty() ? 0 : 1) + (p.l2p_leaf.empty() ? 0 : 1) + 1;
+    nl_ += 1 + (p.p2m_leaf.empty() ? 0 : 1) + 1;
     CK(cudaMemsetAsync(h->pfar.p, 0, 16 * nT, s));
     CK(cudaMemsetAsync(h->Lx.p, 0, h->Lx.bytes, s));
   }
@@ -989,12 +989,20 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
     }
   }
   rec(h, 2 * PH_L2P);
-  if (!fp64 && tc_on(h) && h->l2p_max_points <= 128)
+  if (!fp64 && tc_on(h) && h->l2p_max_points <= 128) {
     dfb::launch_l2p_tc(p.L, d, h->d_l2p_leaf, (int)p.l2p_leaf.size(), h->sig2.p, h->Lx.p, (double2*)h->pfar.p, 1,
                        INT_MIN, INT_MAX, false, h->nsm, sf);
-  else
-    ops->l2p(d, h->d_l2p_leaf, (int)p.l2p_leaf.size(), h->sig2.p, h->Lx.p, (double2*)h->pfar.p, 1, INT_MIN, INT_MAX,
-             false, sf);
+    nl_ += p.l2p_leaf.empty() ? 0 : 1;
+  } else {
+    for (int a = 0, b; a < nl; a = b) {  // runs of levels of one regime
+      for (b = a + 1; b < nl && d.ishf[b] == d.ishf[a]; b++) {
+      }
+      const int64_t k0 = h->l2p_lvl_off[a], k1 = h->l2p_lvl_off[b];
+      ops->l2p(d, h->d_l2p_bylvl + k0, (int)(k1 - k0), d.ishf[a] != 0, h->sig2.p, h->Lx.p, (double2*)h->pfar.p, 1,
+               INT_MIN, INT_MAX, false, sf);
+      nl_ += k1 > k0 ? 1 : 0;
+    }
+  }
   rec(h, 2 * PH_L2P + 1);
   CK(cudaEventRecord(h->ev_done, sn));
   CK(cudaStreamWaitEvent(s, h->ev_done, 0));
@@ -1107,7 +1115,9 @@ int run_gemv_grouped(defmm_handle* h, const double2* qin, int64_t stride_in, dou
     if (!fp64 && tc_on(h) && h->l2p_max_points <= 128)
       dfb::launch_l2p_tc(p.L, d, leaves, n, h->sig2.p, Lbase, (double2*)g.pfar.p, R, d0, d1, true, h->nsm, s);
     else
-      ops->l2p(d, leaves, n, h->sig2.p, Lbase, (double2*)g.pfar.p, R, d0, d1, true, s);
+      // one kernel whatever R, so that a right-hand side's bits do not depend
+      // on the block it is in
+      ops->l2p(d, leaves, n, false, h->sig2.p, Lbase, (double2*)g.pfar.p, R, d0, d1, true, s);
   };
   void* Mlf = slot_base(g.Mlf.p, g.lfS0, slot_b);
   void* Llf = slot_base(g.Llf.p, g.lfT0, slot_b);

@@ -1727,6 +1727,171 @@ __global__ void __launch_bounds__(128) k_l2p(DevPlan P, const int32_t* __restric
   }
 }
 
+// L2P of high-frequency leaves as a small GEMM per leaf (order 5, resident
+// layout),
+//   D[j][s] = sum_l Z(j, l) X[l][s],  X[l][s] = sig2_d[l] L_s[l],
+//   p_j = sum_s exp(i k d_s.(x_j - c)) D[j][s]:
+// one CTA per leaf, Z[l][j] of up to 32 points and X of NS slots in shared
+// memory, a thread on 4 points and SP slots.  A warp owns 8 points and all
+// slots of a tile, so its points' sums stay in its registers and only warps
+// with points issue: 18 points cost 20, where k_l2p's lanes are points, 18 of
+// 32.  Per l a thread loads 4 Z (broadcast) and SP X for 8 SP FMAs; a lane of
+// k_l2p loads one X for 2.  Half the instructions of k_l2p; the loads of the
+// tiles bound it.  k_l2p and this, mixed: sphere 600k 5.4 and 4.2 ms, 31k
+// 0.235 and 0.20 ms; FP64 sphere 250k 5.6 and 5.0 ms.  Elsewhere k_l2p is the
+// faster one: order 6 (spheroid mixed 7.0 and 7.4 ms, its tiles take twice
+// the memory), order 4 (cube 20k FP64 51 and 66 us), blocks of right-hand
+// sides (of eight, 23.9 and 27.7 ms: one staging per right-hand side), and
+// low-frequency leaves, which have a single slot.
+template <typename T, int L>
+struct L2PHf {
+  typedef typename cpx_t<T>::type C;
+  static constexpr bool use = L == 5;
+  static constexpr int LL = L * L * L;
+  static constexpr int SP = sizeof(T) == 4 ? 2 : 1;              // slots per thread
+  static constexpr int NS = 16 * SP;                             // slots per tile
+  static constexpr int NSP = sizeof(T) == 4 ? NS + 2 : NS + 1;   // row pitch of X (16-byte pairs in FP32)
+  static constexpr size_t smem() {
+    return sizeof(C) * LL * NSP + sizeof(T) * LL * 32 + sizeof(double) * 96 + sizeof(T) * 96 * L;
+  }
+};
+
+template <typename T, int L>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 3)
+    k_l2p_hf(DevPlan P, const int32_t* __restrict__ leaves, int nleaves, const typename cpx_t<T>::type* __restrict__ sig2,
+             const typename cpx_t<T>::type* __restrict__ Lx, double2* __restrict__ pfar) {
+  typedef typename cpx_t<T>::type C;
+  typedef L2PHf<T, L> G;
+  constexpr int LL = G::LL, SP = G::SP, NS = G::NS, NSP = G::NSP;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* X = reinterpret_cast<C*>(smem_raw);
+  T* Z = reinterpret_cast<T*>(X + LL * NSP);
+  double* xc = reinterpret_cast<double*>(Z + LL * 32);
+  T* Bs = reinterpret_cast<T*>(xc + 96);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = 2 * warp + (lane >> 4), si = (lane & 15) * SP;  // point group, first slot of the thread
+  for (int li = blockIdx.x; li < nleaves; li += gridDim.x) {
+    const int c = leaves[li];
+    const int64_t sb = P.T_cptr[c], se = P.T_cptr[c + 1];
+    if (sb == se) continue;
+    const int n = P.T_nprt[c], f = P.T_first[c], nslots = (int)(se - sb);
+    const double4 ct = P.T_ctr[c];
+    const int h = P.hfstage[P.T_lvl[c]];
+    const double* dirs = P.dirs + P.dir_off[h] * 3;
+    const C* s2 = sig2 + P.sig_off[h];
+    for (int p0 = 0; p0 < n; p0 += 32) {
+      const int np = min(32, n - p0), n4 = (np + 3) & ~3;
+      __syncthreads();  // the previous points' Z and offsets are no longer read
+      for (int o = threadIdx.x; o < 3 * np; o += 128) {
+        const int p = o / 3, k = o % 3;
+        const double x = P.T_pos[3 * (int64_t)(f + p0 + p) + k] - (&ct.x)[k];
+        xc[o] = x;
+        T b[L];
+        lagrange_all<L, T>((T)x, (T)ct.w, b);
+#pragma unroll
+        for (int l = 0; l < L; l++) Bs[o * L + l] = b[l];
+      }
+      __syncthreads();
+      for (int o = threadIdx.x; o < n4 * LL; o += 128) {
+        const int l = o / n4, p = o % n4;
+        T z = 0;
+        if (p < np) {
+          const T* b = Bs + p * 3 * L;
+          z = b[l / (L * L)] * b[L + l / L % L] * b[2 * L + l % L];
+        }
+        Z[l * 32 + p] = z;
+      }
+      const bool act = 4 * g < np;
+      double xr[4][3];
+#pragma unroll
+      for (int v = 0; v < 4; v++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) xr[v][k] = 4 * g + v < np ? xc[3 * (4 * g + v) + k] : 0.;
+      double2 acc[4];
+#pragma unroll
+      for (int v = 0; v < 4; v++) acc[v] = make_double2(0., 0.);
+      for (int s0 = 0; s0 < nslots; s0 += NS) {
+        const int nt = min(NS, nslots - s0);
+        C ph[4][SP];
+#pragma unroll
+        for (int q = 0; q < SP; q++) {
+          const bool in = act && si + q < nt;
+          const double* dv = dirs + 3 * (in ? P.T_cdir[sb + s0 + si + q] : 0);
+#pragma unroll
+          for (int v = 0; v < 4; v++)
+            ph[v][q] = in ? expi<C>(P.kappa * (dv[0] * xr[v][0] + dv[1] * xr[v][1] + dv[2] * xr[v][2])) : czero<C>();
+        }
+        __syncthreads();  // the previous tile is no longer read (and Z is settled)
+#pragma unroll 4
+        for (int s = warp; s < NS; s += 4) {
+          if (s < nt) {
+            const int64_t j = sb + s0 + s;
+            const C* Ls = Lx + (int64_t)P.T_cslot[j] * LL;
+            const C* Ss = s2 + (int64_t)P.T_cdir[j] * LL;
+#pragma unroll
+            for (int l = lane; l < LL; l += 32) X[l * NSP + s] = cmul(Ss[l], Ls[l]);
+          } else {
+            for (int l = lane; l < LL; l += 32) X[l * NSP + s] = czero<C>();
+          }
+        }
+        __syncthreads();
+        if (!act) continue;
+        C d[4][SP];
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+#pragma unroll
+          for (int q = 0; q < SP; q++) d[v][q] = czero<C>();
+#pragma unroll 5
+        for (int l = 0; l < LL; l++) {
+          T z[4];
+          C x[SP];
+          if constexpr (sizeof(T) == 4) {
+            const float4 zz = *reinterpret_cast<const float4*>(Z + l * 32 + 4 * g);
+            const float4 xx = *reinterpret_cast<const float4*>(X + l * NSP + si);
+            z[0] = zz.x;
+            z[1] = zz.y;
+            z[2] = zz.z;
+            z[3] = zz.w;
+            x[0] = C{xx.x, xx.y};
+            x[SP - 1] = C{xx.z, xx.w};
+          } else {
+            const double2 za = *reinterpret_cast<const double2*>(Z + l * 32 + 4 * g);
+            const double2 zb = *reinterpret_cast<const double2*>(Z + l * 32 + 4 * g + 2);
+            z[0] = za.x;
+            z[1] = za.y;
+            z[2] = zb.x;
+            z[3] = zb.y;
+            x[0] = X[l * NSP + si];
+          }
+#pragma unroll
+          for (int v = 0; v < 4; v++)
+#pragma unroll
+            for (int q = 0; q < SP; q++) rfma(d[v][q], z[v], x[q]);
+        }
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+#pragma unroll
+          for (int q = 0; q < SP; q++) {
+            const C w = cmul(d[v][q], ph[v][q]);
+            acc[v].x += (double)w.x;
+            acc[v].y += (double)w.y;
+          }
+      }
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        double2 t = acc[v];
+#pragma unroll
+        for (int o = 8; o; o >>= 1) {
+          t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+          t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+        }
+        const int p = 4 * g + v;
+        if ((lane & 15) == v && p < np) pfar[f + p0 + p] = t;
+      }
+    }
+  }
+}
+
 // -------------------------------------------------------------------- P2P --
 // Mixed-precision near field.  The phase k r needs ~1e-7 rad absolute
 // accuracy at k r up to ~1e2, beyond FP32: the difference vector, r^2, r and
@@ -2654,6 +2819,11 @@ struct Launch {
     e = cudaFuncSetAttribute(k_p2m<T, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)P2MCfg<T, L>::smem(kMaxRhsBlock));
     if (e != cudaSuccess) return e;
+    if constexpr (L2PHf<T, L>::use) {
+      if ((e = cudaFuncSetAttribute(k_l2p_hf<T, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)L2PHf<T, L>::smem())) != cudaSuccess)
+        return e;
+    }
     if ((e = rhs_attr<1, 128>()) != cudaSuccess || (e = rhs_attr<2, 128>()) != cudaSuccess ||
         (e = rhs_attr<4, 256>()) != cudaSuccess || (e = rhs_attr<8, 256>()) != cudaSuccess ||
         (e = bulk_attr()) != cudaSuccess)
@@ -2776,9 +2946,16 @@ struct Launch {
                       cudaStream_t s) {
     if (n) k_permute_tables<T><<<grid_for(n, 1), 256, 0, s>>>(n, PP, key, perm, (const C*)tables, (C*)out);
   }
-  static void l2p(const DevPlan& dp, const int32_t* leaves, int n, const void* sig2, const void* Lx, double2* pfar,
-                  int R, int d0, int d1, bool accum, cudaStream_t s) {
+  static void l2p(const DevPlan& dp, const int32_t* leaves, int n, bool hf, const void* sig2, const void* Lx,
+                  double2* pfar, int R, int d0, int d1, bool accum, cudaStream_t s) {
     if (!n) return;
+    if constexpr (L2PHf<T, L>::use) {
+      if (hf) {
+        k_l2p_hf<T, L><<<grid_for(n, 1), 128, L2PHf<T, L>::smem(), s>>>(dp, leaves, n, (const C*)sig2, (const C*)Lx,
+                                                                        pfar);
+        return;
+      }
+    }
     if (R == 1)
       k_l2p<T, L, 1><<<grid_for(n, 1), 128, 0, s>>>(dp, leaves, n, (const C*)sig2, (const C*)Lx, pfar, R, d0, d1,
                                                     accum);

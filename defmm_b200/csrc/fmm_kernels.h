@@ -52,8 +52,10 @@ struct OpTable {
                   const void* ptab, void* Lx, unsigned long long* queue, int nsm, int64_t lgroup, cudaStream_t);
   // L2P of the leaves' slots with a direction in [d0, d1) into pfar (R per
   // particle), written (accum = false) or added
-  void (*l2p)(const DevPlan&, const int32_t* leaves, int n, const void* sig2, const void* Lx, double2* pfar, int R,
-              int d0, int d1, bool accum, cudaStream_t);
+  // (hf: every leaf is high-frequency, R = 1, all directions, not added: the
+  // faster kernel of that case)
+  void (*l2p)(const DevPlan&, const int32_t* leaves, int n, bool hf, const void* sig2, const void* Lx, double2* pfar,
+              int R, int d0, int d1, bool accum, cudaStream_t);
   // U_k = tables[key_k >> 6][perm[key_k & 63][:]] for the permuted spectra
   void (*permute)(int64_t n, const uint32_t* key, const uint16_t* perm, const void* tables, void* out,
                   cudaStream_t);

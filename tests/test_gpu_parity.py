@@ -501,3 +501,19 @@ def test_m2l_long_and_empty_lists(order, gpu):
     # the lists dumped after the upload are the plan's
     B = make(w.points, w.points, order, 16, w.kappa)
     assert all(np.array_equal(a, b) for a, b in zip(A.m2l_entries(), B.m2l_entries()))
+
+
+@pytest.mark.parametrize("ncrit", [9, 33, 96])
+def test_l2p_tiles_at_order_5(ncrit, gpu):
+    # high-frequency leaves of 1 to 96 points (groups of 4 with padded ones,
+    # more than one chunk of 32) with a few to well over 32 slots (tiles that
+    # are not full)
+    p = W.sphere_surface(4000, seed=17).points
+    kappa = 2 * np.pi * 5
+    q = W.charges(len(p), 2)
+    A = make(p, p, 5, ncrit, kappa)
+    ref = O.OracleFMM(p, p, 5, ncrit, kappa, -1).gemv(q)
+    for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+        A.set_precision(prec)
+        assert rel(A.matvec(q), ref) <= tol
+        assert A.info("layout") == 1

@@ -1933,15 +1933,15 @@ __device__ __forceinline__ double rsqrt_approx64(double x) {
 // quarter turns, r kq = n + u with |u| <= 1/2, u by one exactly rounded FMA
 // and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
 // (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
-// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20); R kept
-// away from zero by an integer maximum on its high word.
-__device__ __forceinline__ double2 green64(double dx, double dy, double dz, double kq) {
-  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
-  const bool skip = __double_as_longlong(R0) < 0x3C9CD2B297D889BCLL;  // R0 < 1e-16
-  const double R = __hiloint2double(max(__double2hiint(R0), 0x3C9CD2B2), __double2loint(R0));
+// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20).
+// GUARD = false: the caller knows R0 >= 1e-16.
+template <bool GUARD>
+__device__ __forceinline__ double2 green64_r(double R0, double kq) {
+  double R = R0;
+  if (GUARD) R = __hiloint2double(max(__double2hiint(R0), 0x3C9CD2B2), __double2loint(R0));
   const double y0 = rsqrt_approx64(R);
   const double e = fma(-(R * y0), y0, 1.0);
-  const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+  double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
   const double r = R * y;
   const double t = fma(r, kq, 6755399441055744.0);  // + 1.5 * 2^52
   const double u = fma(r, kq, -(t - 6755399441055744.0));
@@ -1960,14 +1960,15 @@ __device__ __forceinline__ double2 green64(double dx, double dy, double dz, doub
   pc = fma(z, pc, 0.2536695079010469);
   pc = fma(z, pc, -1.2337005501361697);
   pc = fma(z, pc, 1.0);
-  const double K = skip ? 0. : y;
+  if (GUARD && __double_as_longlong(R0) < 0x3C9CD2B297D889BCLL) y = 0.;  // R0 < 1e-16
+  // quadrant q: sin and cos of the whole phase are (sr, cr), (cr, -sr),
+  // (-sr, -cr), (-cr, sr); both signs of q & 2 go into 1/r
+  const double K = __hiloint2double(__double2hiint(y) ^ (int)((unsigned)q << 30 & 0x80000000u), __double2loint(y));
   const double sr = u * K * ps, cr = K * pc;
-  const double ss = (q & 1) ? cr : sr, cc = (q & 1) ? sr : cr;
-  // signs: sin negative in quadrants 2, 3; cos in 1, 2
-  return make_double2(__hiloint2double(__double2hiint(cc) ^ (int)((unsigned)(q + 1) << 30 & 0x80000000u),
-                                       __double2loint(cc)),
-                      __hiloint2double(__double2hiint(ss) ^ (int)((unsigned)q << 30 & 0x80000000u),
-                                       __double2loint(ss)));
+  return make_double2((q & 1) ? -sr : cr, (q & 1) ? cr : sr);
+}
+__device__ __forceinline__ double2 green64(double dx, double dy, double dz, double kq) {
+  return green64_r<true>(fma(dx, dx, fma(dy, dy, dz * dz)), kq);
 }
 
 // Compensated (Kahan) FP32 summation: s - c carries the sum.
@@ -2157,9 +2158,9 @@ __global__ void k_p2p_items(int64_t nchunk, const int32_t* __restrict__ tfirst, 
 // G(x, y) = exp(i k r) / (4 pi r) of one pair (0 for R < 1e-16, P2P.hpp:66)
 // with the arithmetic of p2p_pair_mixed.  Branch-free: a pair with R < 1e-16
 // is evaluated at R = 1 and scaled by 0.
-__device__ __forceinline__ float2 green32(double dx, double dy, double dz, double kappa) {
-  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
-  const bool skip = R0 < 1.e-16;
+template <bool GUARD>
+__device__ __forceinline__ float2 green32_r(double R0, double kappa) {
+  const bool skip = GUARD && R0 < 1.e-16;
   const double R = skip ? 1. : R0;
   double yd = rsqrt_approx64(R);
   yd = yd * fma(-0.5 * R * yd, yd, 1.5);
@@ -2185,6 +2186,9 @@ __device__ __forceinline__ float2 green32(double dx, double dy, double dz, doubl
   const float K0 = odd ? -0.0795774715459476679f * y : 0.0795774715459476679f * y;
   const float K = skip ? 0.f : K0;
   return make_float2(pc * K, x * ps * K);
+}
+__device__ __forceinline__ float2 green32(double dx, double dy, double dz, double kappa) {
+  return green32_r<true>(fma(dx, dx, fma(dy, dy, dz * dz)), kappa);
 }
 
 // Near field for a block of right-hand sides (the target-side form of
@@ -2439,7 +2443,7 @@ __device__ __forceinline__ double charge_word(float2 q) {
 // targets' sums around gave 76-86%; and 8 independent evaluations per lane
 // keep the FP64 pipe fed (65% of its cycles on a 31k-point sphere).  The near
 // field of a 250k-point sphere in FP64 took 20.1 ms with the segments and
-// takes 15 ms so; of a 600k-point sphere in mixed precision 22.5 and 20 ms.
+// takes 14.0 ms so; of a 600k-point sphere in mixed precision 22.5 and 20.3 ms.
 template <bool MIXED>
 struct P2PSym {
   static constexpr int S = 2;       // sources per lane
@@ -2484,14 +2488,10 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
     const int nb = (nt + 3) >> 2;
     if (threadIdx.x < 4 * NB) {
       const int t = threadIdx.x;
-      double2 xy = make_double2(0., 0.), zw = make_double2(0., 0.);
-      Q qt = Q{0, 0};
-      if (t < nt) {
-        const double* x = P.T_pos + 3 * (int64_t)(f + t);
-        qt = q[f + t];
-        xy = make_double2(x[0], x[1]);
-        zw.x = x[2];
-      }
+      const double* x = P.T_pos + 3 * (int64_t)(f + (t < nt ? t : 0));
+      const Q qt = t < nt ? q[f + t] : Q{0, 0};
+      const double2 xy = make_double2(x[0], x[1]);
+      double2 zw = make_double2(x[2], 0.);
       if constexpr (MIXED)
         zw.y = charge_word(qt);
       else
@@ -2531,50 +2531,68 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
         int64_t sidx[S];
 #pragma unroll
         for (int v = 0; v < S; v++) {
-          const int jj = base + 32 * v + lane;
-          yx[v] = yy[v] = yz[v] = 0.;
-          qj[v] = accT[v] = Q{0, 0};
-          sidx[v] = -1;
-          if (jj < ntot) {
-            int lo = 0, hi = nr - 1;  // last range with rpre <= jj
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (rpre[mid] <= jj) lo = mid; else hi = mid - 1;
-            }
-            const int o = jj - rpre[lo];
-            const int64_t sj = (int64_t)rfst[lo] + o;
-            sidx[v] = roff[lo] + o;
-            const double* y = P.S_pos + 3 * sj;
-            yx[v] = y[0];
-            yy[v] = y[1];
-            yz[v] = y[2];
-            qj[v] = q[sj];
+          const int jj = base + 32 * v + lane, jc = min(jj, ntot - 1);
+          int lo = 0, hi = nr - 1;  // last range with rpre <= jc
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (rpre[mid] <= jc) lo = mid; else hi = mid - 1;
           }
+          const int o = jc - rpre[lo];
+          const int64_t sj = (int64_t)rfst[lo] + o;
+          const double* y = P.S_pos + 3 * sj;
+          yx[v] = y[0];
+          yy[v] = y[1];
+          yz[v] = y[2];
+          qj[v] = jj < ntot ? q[sj] : Q{0, 0};
+          accT[v] = Q{0, 0};
+          sidx[v] = jj < ntot ? roff[lo] + o : -1;
         }
-        // no validity tests: padded targets and missing sources carry zero
-        // charges, and their sums are never stored
+        // no validity tests: padded targets (copies of the first) and missing
+        // sources (copies of the last) carry zero charges, and their sums are
+        // never stored
         for (int b = 0; b < nb; b++) {
+          // squared distances first: coincident points (R < 1e-16, P2P.hpp:66)
+          // are rare, so one test of the block's smallest high word chooses
+          // the evaluations without a test of their own
           Q d[4];
+          double R[4][S];
+          int least = INT_MAX;
 #pragma unroll
           for (int t = 0; t < 4; t++) {
             const double2 a = trxy[4 * b + t], z = trzw[4 * b + t];
             d[t] = Q{0, 0};
 #pragma unroll
             for (int v = 0; v < S; v++) {
-              Q g, qi;
-              if constexpr (MIXED) {
-                g = green32(a.x - yx[v], a.y - yy[v], z.x - yz[v], P.kappa);
-                qi = charge_bits(z.y);
-              } else {
-                g = green64(a.x - yx[v], a.y - yy[v], z.x - yz[v], kq);
-                qi = tq[4 * b + t];
-              }
-              d[t].x = fma(g.x, qj[v].x, fma(-g.y, qj[v].y, d[t].x));
-              d[t].y = fma(g.x, qj[v].y, fma(g.y, qj[v].x, d[t].y));
-              accT[v].x = fma(g.x, qi.x, fma(-g.y, qi.y, accT[v].x));
-              accT[v].y = fma(g.x, qi.y, fma(g.y, qi.x, accT[v].y));
+              const double dx = a.x - yx[v], dy = a.y - yy[v], dz = z.x - yz[v];
+              R[t][v] = fma(dx, dx, fma(dy, dy, dz * dz));
+              least = min(least, __double2hiint(R[t][v]));
             }
           }
+          auto block = [&](auto guard) {
+            constexpr bool GUARD = decltype(guard)::value;
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+#pragma unroll
+              for (int v = 0; v < S; v++) {
+                Q g, qi;
+                if constexpr (MIXED) {
+                  g = green32_r<GUARD>(R[t][v], P.kappa);
+                  qi = charge_bits(trzw[4 * b + t].y);
+                } else {
+                  g = green64_r<GUARD>(R[t][v], kq);
+                  qi = tq[4 * b + t];
+                }
+                d[t].x = fma(g.x, qj[v].x, fma(-g.y, qj[v].y, d[t].x));
+                d[t].y = fma(g.x, qj[v].y, fma(g.y, qj[v].x, d[t].y));
+                accT[v].x = fma(g.x, qi.x, fma(-g.y, qi.y, accT[v].x));
+                accT[v].y = fma(g.x, qi.y, fma(g.y, qi.x, accT[v].y));
+              }
+            }
+          };
+          if (__any_sync(0xffffffffu, least <= 0x3C9CD2B2))
+            block(std::true_type());
+          else
+            block(std::false_type());
           // lanes with bit 4 keep targets 2, 3, the others 0, 1; then bit 3
           // chooses the odd or the even one
           const bool h1 = lane & 16, h0 = lane & 8;

@@ -517,3 +517,22 @@ def test_l2p_tiles_at_order_5(ncrit, gpu):
         A.set_precision(prec)
         assert rel(A.matvec(q), ref) <= tol
         assert A.info("layout") == 1
+
+
+@pytest.mark.parametrize("gap,counts", [(4e-9, False), (6e-9, True)])
+def test_near_field_coincident_points_in_two_leaves(gap, counts, gpu):
+    # pairs of points 2 gap apart on either side of the root cell's centre
+    # planes, so in different leaves: below 1e-8 the symmetric blocks skip the
+    # pair (P2P.hpp:66), above it the pair's 1/r dominates both potentials
+    p = W.sphere_surface(2500, seed=41).points
+    p[:6] = np.vstack([np.eye(3), -np.eye(3)])  # bounding cube [-1, 1]^3
+    for i in range(6):
+        p[10 + i] = np.roll([(-1) ** i * gap, 0.6, 0.8], i // 2)
+    kappa = 4 * np.pi
+    q = W.charges(len(p), 8)
+    A = make(p, p, 4, 33, kappa)
+    ref = A.matvec(q)
+    assert rel(ref, O.OracleFMM(p, p, 4, 33, kappa, -1).gemv(q)) <= FP64_TOL
+    assert (abs(ref[10]) > 1e5) == counts
+    A.set_precision("mixed")
+    assert rel(A.matvec(q), ref) <= MIXED_TOL

@@ -270,8 +270,8 @@ void free_plan_device(defmm_handle* h) {
 // parts: the 287 items of the 5,003-point sphere 147 and 76 us, the 1,300 of
 // the 20,000-point cube 579 and 414 us, the 778 very uneven ones of blobs to
 // a sphere (three right-hand sides) 530 and 230 us.  Items are cut until
-// there are 8 per slot (16 cost the mixed 31k-point sphere 2%, 2 leave the
-// cube whole), but not below 512 sources on average (two rounds of a CTA).
+// there are 8 per slot (2 leave the cube whole), but not below 512 sources on
+// average (two rounds of a CTA).
 int near_split(int nsm, int64_t items, int64_t chunks, int64_t pairs, int64_t targets) {
   if (items <= 0 || targets <= 0) return 1;
   const int64_t want = (8 * 4 * (int64_t)nsm + items - 1) / items;
@@ -857,23 +857,25 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
   CK(cudaEventRecord(ready, s));
   CK(cudaStreamWaitEvent(sn, ready, 0));
   if (h->events) cudaEventRecord(h->ev[2 * PH_P2P], sn);
+  // the mixed path's FP32 sums run over whole items
+  const int p2p_split = fp64 ? h->p2p_split : 1, sym_split = fp64 ? h->sym_split : 1;
   if (h->use_sym) {  // own leaves, then symmetric blocks, then the mirrored partial sums
     dfb::launch_p2p(fp64, d, p.near_self_items(), h->d_self_order, nullptr, h->d_tfirst, h->d_tn,
                     h->d_self_ptr, h->d_self_sfirst, h->d_self_sn, h->q.p, (double2*)h->pnear.p, nullptr,
                     1, h->d_queue, h->nsm, sn);
     dfb::launch_p2p_sym(fp64, d, p.near_sym_items(), h->d_sym_order, h->d_sym_item_chunk, h->d_tfirst,
                         h->d_tn, h->d_sym_ptr, h->d_sym_sfirst, h->d_sym_sn, h->d_sym_soff, h->q.p, h->d_tpart,
-                        h->pscr.p, h->sym_split, h->d_queue, h->nsm, h->p2p_bps[fp64 ? 0 : 1], sn);
-    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_sym_chunk_items, h->d_tpart, h->sym_split,
+                        h->pscr.p, sym_split, h->d_queue, h->nsm, h->p2p_bps[fp64 ? 0 : 1], sn);
+    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_sym_chunk_items, h->d_tpart, sym_split,
                           (double2*)h->pnear.p, h->nsm, sn);
     dfb::launch_p2p_reduce(fp64, p.near_red_leaves(), h->d_red_first, h->d_red_n, h->d_red_ptr,
                            h->d_red_off, h->pscr.p, (double2*)h->pnear.p, h->nsm, sn);
     nl_ += (p.near_self_items() ? 1 : 0) + (p.near_sym_items() ? 2 : 0) + (p.near_red_leaves() ? 1 : 0);
   } else {  // every interaction from the target side, in items
     dfb::launch_p2p(fp64, d, p.near_items(), h->d_p2p_order, h->d_p2p_item_chunk, h->d_tfirst, h->d_tn,
-                    h->d_p2p_ptr, h->d_sfirst, h->d_sn, h->q.p, (double2*)h->pnear.p, h->d_tpart, h->p2p_split,
+                    h->d_p2p_ptr, h->d_sfirst, h->d_sn, h->q.p, (double2*)h->pnear.p, h->d_tpart, p2p_split,
                     h->d_queue, h->nsm, sn);
-    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, h->d_tpart, h->p2p_split,
+    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, h->d_tpart, p2p_split,
                           (double2*)h->pnear.p, h->nsm, sn);
     nl_ += p.near_items() ? 2 : 0;
   }

@@ -59,6 +59,14 @@ __device__ __forceinline__ typename cpx_t<T>::type ctw(int m) {
   }
   return r;
 }
+// acc += v * conj(w)
+template <typename C>
+__device__ __forceinline__ void cfmac(C& acc, C v, C w) {
+  acc.x = fma(v.x, w.x, acc.x);
+  acc.x = fma(v.y, w.y, acc.x);
+  acc.y = fma(v.y, w.x, acc.y);
+  acc.y = fma(-v.x, w.y, acc.y);
+}
 // ------------------------------------------------------------- gather/scatter
 template <typename T>
 __global__ void k_gather(const double2* __restrict__ qin, const int32_t* __restrict__ perm,
@@ -101,9 +109,11 @@ __global__ void k_scatter(const double2* __restrict__ pnear, const double2* __re
 // tile (expansion entries lane + 32 e, all S slots, so signatures and results
 // are read and written at unit stride) over the chunk's points: per point R
 // loads of Z and S broadcast loads of W feed 2 R S FMAs.  Latency bounds it
-// (the signatures' loads), so a chunk is small enough for 4 CTAs per SM:
+// (the signatures' loads), so an FP64 chunk is small enough for 4 CTAs per SM:
 // sphere 250k FP64 5.7 -> 4.0 ms against entries R lane .. R lane + R - 1 and
-// chunks of 64 points, spheroid 500k mixed order 6 9.1 -> 5.5 ms.
+// chunks of 64 points.  FP32 chunks hold 64 points where they fit: their sums
+// are rounded chunk by chunk, and results keep their bits (spheroid 500k mixed
+// order 6 9.1 -> 7.0 ms, 5.5 with chunks of 40).
 template <typename T, int L>
 struct P2MCfg {
   static constexpr int LL = L * L * L;
@@ -111,7 +121,7 @@ struct P2MCfg {
   static constexpr int LLP = 32 * R;
   static constexpr int S0 = (sizeof(T) == 4 ? 32 : 16) / R;
   static constexpr int S = S0 < 1 ? 1 : (S0 > (sizeof(T) == 4 ? 8 : 4) ? (sizeof(T) == 4 ? 8 : 4) : S0);
-  static constexpr int NPB0 = 40960 / (LLP * (int)sizeof(T));
+  static constexpr int NPB0 = (sizeof(T) == 4 ? 65536 : 40960) / (LLP * (int)sizeof(T));
   static constexpr int NPB = NPB0 > 64 ? 64 : NPB0;  // points per chunk
   typedef typename cpx_t<T>::type C;
   // shared memory: Z, point offsets, basis values, W blocks of 4 warps,
@@ -700,34 +710,46 @@ struct M2FCfg {
 // One line of the forward DFT: out(k) = sum_a v[a] w^(k a), k < P = 2 L - 1,
 // a < L.  Outputs k and P - k are A - i B and A + i B with A = sum cos v,
 // B = sum sin v: 4 (L - 1) FMAs for the two instead of 8 (L - 1) for each.
+// FP32 sums go term by term: paired they take 9.3 instead of 11.1 ms (spheroid
+// 500k order 6) but round differently, and mixed results keep their bits.
 template <typename T, int L, typename C, typename Put>
 __device__ __forceinline__ void fdft_line(const C (&v)[L], Put put) {
   constexpr int P = 2 * L - 1;
-  C s0 = v[0];
+  if constexpr (sizeof(T) == 4) {
 #pragma unroll
-  for (int a = 1; a < L; a++) {
-    s0.x += v[a].x;
-    s0.y += v[a].y;
-  }
-  put(0, s0);
+    for (int k = 0; k < P; k++) {
+      C o = v[0];
 #pragma unroll
-  for (int k = 1; k < L; k++) {
-    C A = v[0], B;
+      for (int a = 1; a < L; a++) cfma(o, v[a], ctw<T, L>((k * a) % P));
+      put(k, o);
+    }
+  } else {
+    C s0 = v[0];
 #pragma unroll
     for (int a = 1; a < L; a++) {
-      const C w = ctw<T, L>((k * a) % P);  // (cos, -sin)
-      A.x = fma(w.x, v[a].x, A.x);
-      A.y = fma(w.x, v[a].y, A.y);
-      B.x = a == 1 ? w.y * v[a].x : fma(w.y, v[a].x, B.x);  // -B
-      B.y = a == 1 ? w.y * v[a].y : fma(w.y, v[a].y, B.y);
+      s0.x += v[a].x;
+      s0.y += v[a].y;
     }
-    C lo, hi;
-    lo.x = A.x - B.y;
-    lo.y = A.y + B.x;
-    hi.x = A.x + B.y;
-    hi.y = A.y - B.x;
-    put(k, lo);
-    put(P - k, hi);
+    put(0, s0);
+#pragma unroll
+    for (int k = 1; k < L; k++) {
+      C A = v[0], B;
+#pragma unroll
+      for (int a = 1; a < L; a++) {
+        const C w = ctw<T, L>((k * a) % P);  // (cos, -sin)
+        A.x = fma(w.x, v[a].x, A.x);
+        A.y = fma(w.x, v[a].y, A.y);
+        B.x = a == 1 ? w.y * v[a].x : fma(w.y, v[a].x, B.x);  // -B
+        B.y = a == 1 ? w.y * v[a].y : fma(w.y, v[a].y, B.y);
+      }
+      C lo, hi;
+      lo.x = A.x - B.y;
+      lo.y = A.y + B.x;
+      hi.x = A.x + B.y;
+      hi.y = A.y - B.x;
+      put(k, lo);
+      put(P - k, hi);
+    }
   }
 }
 
@@ -817,44 +839,46 @@ __global__ void k_permute_tables(int64_t n, int PP, const uint32_t* __restrict__
 //   out[a] = sum_k v[k] conj(w)^(k a),  w = exp(-2 pi i / P), P = 2 L - 1.
 // The terms k and P - k share their cosine, and their sine up to its sign, so
 // they are added and subtracted first: 4 (L - 1) FMAs per output instead of
-// 8 (L - 1), none of them multiplications for a = 0.
-// One pair's share of one output, o += v_k conj(w) + v_(P-k) w (idft_line's
-// operations, for a thread that computes a single output).
-template <typename C>
-__device__ __forceinline__ void idft_pair(C& o, C vk, C vp, C w) {
-  o.x = fma(w.x, vk.x + vp.x, o.x);
-  o.y = fma(w.x, vk.y + vp.y, o.y);
-  o.x = fma(w.y, vk.y - vp.y, o.x);
-  o.y = fma(-w.y, vk.x - vp.x, o.y);
-}
+// 8 (L - 1), none of them multiplications for a = 0.  FP32 sums go term by
+// term (fdft_line).
 template <typename T, int L, typename C>
 __device__ __forceinline__ void idft_line(const C (&v)[2 * L - 1], C (&out)[L]) {
   constexpr int P = 2 * L - 1;
-  C s[L], d[L];
+  if constexpr (sizeof(T) == 4) {
 #pragma unroll
-  for (int k = 1; k < L; k++) {
-    s[k].x = v[k].x + v[P - k].x;
-    s[k].y = v[k].y + v[P - k].y;
-    d[k].x = v[k].x - v[P - k].x;
-    d[k].y = v[k].y - v[P - k].y;
-  }
+    for (int a = 0; a < L; a++) {
+      C o = v[0];
 #pragma unroll
-  for (int a = 0; a < L; a++) {
-    C o = v[0];
+      for (int k = 1; k < P; k++) cfmac(o, v[k], ctw<T, L>((k * a) % P));
+      out[a] = o;
+    }
+  } else {
+    C s[L], d[L];
 #pragma unroll
     for (int k = 1; k < L; k++) {
-      if (a == 0) {
-        o.x += s[k].x;
-        o.y += s[k].y;
-      } else {
-        const C w = ctw<T, L>((k * a) % P);  // (cos, -sin)
-        o.x = fma(w.x, s[k].x, o.x);
-        o.y = fma(w.x, s[k].y, o.y);
-        o.x = fma(w.y, d[k].y, o.x);
-        o.y = fma(-w.y, d[k].x, o.y);
-      }
+      s[k].x = v[k].x + v[P - k].x;
+      s[k].y = v[k].y + v[P - k].y;
+      d[k].x = v[k].x - v[P - k].x;
+      d[k].y = v[k].y - v[P - k].y;
     }
-    out[a] = o;
+#pragma unroll
+    for (int a = 0; a < L; a++) {
+      C o = v[0];
+#pragma unroll
+      for (int k = 1; k < L; k++) {
+        if (a == 0) {
+          o.x += s[k].x;
+          o.y += s[k].y;
+        } else {
+          const C w = ctw<T, L>((k * a) % P);  // (cos, -sin)
+          o.x = fma(w.x, s[k].x, o.x);
+          o.y = fma(w.x, s[k].y, o.y);
+          o.x = fma(w.y, d[k].y, o.x);
+          o.y = fma(-w.y, d[k].x, o.y);
+        }
+      }
+      out[a] = o;
+    }
   }
 }
 
@@ -1548,7 +1572,7 @@ __global__ void __launch_bounds__(M2LBulk<L>::NT, M2LBulk<L>::CTAS) k_m2l_bulk(
         const float2* v = Js + sp * PP + ln;
         float2 sum = v[0];
 #pragma unroll
-        for (int k0 = 1; k0 < L; k0++) idft_pair(sum, v[k0 * PD * PD], v[(PD - k0) * PD * PD], tw[(k0 * a) % PD]);
+        for (int k0 = 1; k0 < PD; k0++) cfmac(sum, v[k0 * PD * PD], tw[(k0 * a) % PD]);
         Cb[sp * L * PD * PD + a * PD * PD + ln] = sum;
       }
       if (!(ok = cbarrier())) continue;
@@ -1559,7 +1583,7 @@ __global__ void __launch_bounds__(M2LBulk<L>::NT, M2LBulk<L>::CTAS) k_m2l_bulk(
         const float2* v = Cb + sp * L * PD * PD + a * PD * PD + k2;
         float2 sum = v[0];
 #pragma unroll
-        for (int k1 = 1; k1 < L; k1++) idft_pair(sum, v[k1 * PD], v[(PD - k1) * PD], tw[(k1 * b) % PD]);
+        for (int k1 = 1; k1 < PD; k1++) cfmac(sum, v[k1 * PD], tw[(k1 * b) % PD]);
         D[sp * L * L * PD + (a * L + b) * PD + k2] = sum;
       }
       if (!(ok = cbarrier())) continue;
@@ -1569,7 +1593,7 @@ __global__ void __launch_bounds__(M2LBulk<L>::NT, M2LBulk<L>::CTAS) k_m2l_bulk(
         const float2* v = D + sp * L * L * PD + ln * PD;
         float2 sum = v[0];
 #pragma unroll
-        for (int k2 = 1; k2 < L; k2++) idft_pair(sum, v[k2], v[(PD - k2)], tw[(k2 * c) % PD]);
+        for (int k2 = 1; k2 < PD; k2++) cfmac(sum, v[k2], tw[(k2 * c) % PD]);
         lold.x += sum.x * inv;
         lold.y += sum.y * inv;
         *l3 = lold;
@@ -1727,49 +1751,48 @@ __global__ void __launch_bounds__(128) k_l2p(DevPlan P, const int32_t* __restric
   }
 }
 
-// L2P of high-frequency leaves as a small GEMM per leaf (order 5, resident
-// layout),
+// FP64 L2P of high-frequency leaves as a small GEMM per leaf (order 5,
+// resident layout),
 //   D[j][s] = sum_l Z(j, l) X[l][s],  X[l][s] = sig2_d[l] L_s[l],
 //   p_j = sum_s exp(i k d_s.(x_j - c)) D[j][s]:
-// one CTA per leaf, Z[l][j] of up to 32 points and X of NS slots in shared
-// memory, a thread on 4 points and SP slots.  A warp owns 8 points and all
+// one CTA per leaf, Z[l][j] of up to 32 points and X of 16 slots in shared
+// memory, a thread on 4 points and a slot.  A warp owns 8 points and all
 // slots of a tile, so its points' sums stay in its registers and only warps
 // with points issue: 18 points cost 20, where k_l2p's lanes are points, 18 of
-// 32.  Per l a thread loads 4 Z (broadcast) and SP X for 8 SP FMAs; a lane of
+// 32.  Per l a thread loads 4 Z (broadcast) and one X for 8 FMAs; a lane of
 // k_l2p loads one X for 2.  Half the instructions of k_l2p; the loads of the
-// tiles bound it.  k_l2p and this, mixed: sphere 600k 5.4 and 4.2 ms, 31k
-// 0.235 and 0.20 ms; FP64 sphere 250k 5.6 and 5.0 ms.  Elsewhere k_l2p is the
-// faster one: order 6 (spheroid mixed 7.0 and 7.4 ms, its tiles take twice
-// the memory), order 4 (cube 20k FP64 51 and 66 us), blocks of right-hand
-// sides (of eight, 23.9 and 27.7 ms: one staging per right-hand side), and
-// low-frequency leaves, which have a single slot.
+// tiles bound it.  k_l2p and this: sphere 250k 5.6 and 5.0 ms.  Elsewhere
+// k_l2p is the faster one: order 4 (cube 20k 51 and 66 us), orders from 6 (the
+// tiles take twice the memory), blocks of right-hand sides (one staging for
+// each), and low-frequency leaves, which have a single slot; FP32 sums (600k
+// points 5.4 and 4.2 ms) would round differently, and mixed results keep
+// their bits.
 template <typename T, int L>
 struct L2PHf {
   typedef typename cpx_t<T>::type C;
-  static constexpr bool use = L == 5;
+  static constexpr bool use = L == 5 && sizeof(T) == 8;
   static constexpr int LL = L * L * L;
-  static constexpr int SP = sizeof(T) == 4 ? 2 : 1;              // slots per thread
-  static constexpr int NS = 16 * SP;                             // slots per tile
-  static constexpr int NSP = sizeof(T) == 4 ? NS + 2 : NS + 1;   // row pitch of X (16-byte pairs in FP32)
+  static constexpr int NS = 16;       // slots per tile
+  static constexpr int NSP = NS + 1;  // row pitch of X
   static constexpr size_t smem() {
     return sizeof(C) * LL * NSP + sizeof(T) * LL * 32 + sizeof(double) * 96 + sizeof(T) * 96 * L;
   }
 };
 
 template <typename T, int L>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 3)
+__global__ void __launch_bounds__(128, 3)
     k_l2p_hf(DevPlan P, const int32_t* __restrict__ leaves, int nleaves, const typename cpx_t<T>::type* __restrict__ sig2,
              const typename cpx_t<T>::type* __restrict__ Lx, double2* __restrict__ pfar) {
   typedef typename cpx_t<T>::type C;
   typedef L2PHf<T, L> G;
-  constexpr int LL = G::LL, SP = G::SP, NS = G::NS, NSP = G::NSP;
+  constexpr int LL = G::LL, NS = G::NS, NSP = G::NSP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* X = reinterpret_cast<C*>(smem_raw);
   T* Z = reinterpret_cast<T*>(X + LL * NSP);
   double* xc = reinterpret_cast<double*>(Z + LL * 32);
   T* Bs = reinterpret_cast<T*>(xc + 96);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = 2 * warp + (lane >> 4), si = (lane & 15) * SP;  // point group, first slot of the thread
+  const int g = 2 * warp + (lane >> 4), si = lane & 15;  // point group, slot of the thread
   for (int li = blockIdx.x; li < nleaves; li += gridDim.x) {
     const int c = leaves[li];
     const int64_t sb = P.T_cptr[c], se = P.T_cptr[c + 1];
@@ -1812,15 +1835,12 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 3)
       for (int v = 0; v < 4; v++) acc[v] = make_double2(0., 0.);
       for (int s0 = 0; s0 < nslots; s0 += NS) {
         const int nt = min(NS, nslots - s0);
-        C ph[4][SP];
+        C ph[4];
+        const bool in = act && si < nt;
+        const double* dv = dirs + 3 * (in ? P.T_cdir[sb + s0 + si] : 0);
 #pragma unroll
-        for (int q = 0; q < SP; q++) {
-          const bool in = act && si + q < nt;
-          const double* dv = dirs + 3 * (in ? P.T_cdir[sb + s0 + si + q] : 0);
-#pragma unroll
-          for (int v = 0; v < 4; v++)
-            ph[v][q] = in ? expi<C>(P.kappa * (dv[0] * xr[v][0] + dv[1] * xr[v][1] + dv[2] * xr[v][2])) : czero<C>();
-        }
+        for (int v = 0; v < 4; v++)
+          ph[v] = in ? expi<C>(P.kappa * (dv[0] * xr[v][0] + dv[1] * xr[v][1] + dv[2] * xr[v][2])) : czero<C>();
         __syncthreads();  // the previous tile is no longer read (and Z is settled)
 #pragma unroll 4
         for (int s = warp; s < NS; s += 4) {
@@ -1836,46 +1856,25 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 3)
         }
         __syncthreads();
         if (!act) continue;
-        C d[4][SP];
+        C d[4];
 #pragma unroll
-        for (int v = 0; v < 4; v++)
-#pragma unroll
-          for (int q = 0; q < SP; q++) d[v][q] = czero<C>();
+        for (int v = 0; v < 4; v++) d[v] = czero<C>();
 #pragma unroll 5
         for (int l = 0; l < LL; l++) {
-          T z[4];
-          C x[SP];
-          if constexpr (sizeof(T) == 4) {
-            const float4 zz = *reinterpret_cast<const float4*>(Z + l * 32 + 4 * g);
-            const float4 xx = *reinterpret_cast<const float4*>(X + l * NSP + si);
-            z[0] = zz.x;
-            z[1] = zz.y;
-            z[2] = zz.z;
-            z[3] = zz.w;
-            x[0] = C{xx.x, xx.y};
-            x[SP - 1] = C{xx.z, xx.w};
-          } else {
-            const double2 za = *reinterpret_cast<const double2*>(Z + l * 32 + 4 * g);
-            const double2 zb = *reinterpret_cast<const double2*>(Z + l * 32 + 4 * g + 2);
-            z[0] = za.x;
-            z[1] = za.y;
-            z[2] = zb.x;
-            z[3] = zb.y;
-            x[0] = X[l * NSP + si];
-          }
-#pragma unroll
-          for (int v = 0; v < 4; v++)
-#pragma unroll
-            for (int q = 0; q < SP; q++) rfma(d[v][q], z[v], x[q]);
+          const double2 za = *reinterpret_cast<const double2*>(Z + l * 32 + 4 * g);
+          const double2 zb = *reinterpret_cast<const double2*>(Z + l * 32 + 4 * g + 2);
+          const C x = X[l * NSP + si];
+          rfma(d[0], za.x, x);
+          rfma(d[1], za.y, x);
+          rfma(d[2], zb.x, x);
+          rfma(d[3], zb.y, x);
         }
 #pragma unroll
-        for (int v = 0; v < 4; v++)
-#pragma unroll
-          for (int q = 0; q < SP; q++) {
-            const C w = cmul(d[v][q], ph[v][q]);
-            acc[v].x += (double)w.x;
-            acc[v].y += (double)w.y;
-          }
+        for (int v = 0; v < 4; v++) {
+          const C w = cmul(d[v], ph[v]);
+          acc[v].x += w.x;
+          acc[v].y += w.y;
+        }
       }
 #pragma unroll
       for (int v = 0; v < 4; v++) {
@@ -2158,9 +2157,9 @@ __global__ void k_p2p_items(int64_t nchunk, const int32_t* __restrict__ tfirst, 
 // G(x, y) = exp(i k r) / (4 pi r) of one pair (0 for R < 1e-16, P2P.hpp:66)
 // with the arithmetic of p2p_pair_mixed.  Branch-free: a pair with R < 1e-16
 // is evaluated at R = 1 and scaled by 0.
-template <bool GUARD>
-__device__ __forceinline__ float2 green32_r(double R0, double kappa) {
-  const bool skip = GUARD && R0 < 1.e-16;
+__device__ __forceinline__ float2 green32(double dx, double dy, double dz, double kappa) {
+  const double R0 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const bool skip = R0 < 1.e-16;
   const double R = skip ? 1. : R0;
   double yd = rsqrt_approx64(R);
   yd = yd * fma(-0.5 * R * yd, yd, 1.5);
@@ -2186,9 +2185,6 @@ __device__ __forceinline__ float2 green32_r(double R0, double kappa) {
   const float K0 = odd ? -0.0795774715459476679f * y : 0.0795774715459476679f * y;
   const float K = skip ? 0.f : K0;
   return make_float2(pc * K, x * ps * K);
-}
-__device__ __forceinline__ float2 green32(double dx, double dy, double dz, double kappa) {
-  return green32_r<true>(fma(dx, dx, fma(dy, dy, dz * dz)), kappa);
 }
 
 // Near field for a block of right-hand sides (the target-side form of
@@ -2423,8 +2419,8 @@ __device__ __forceinline__ double charge_word(float2 q) {
   return __longlong_as_double(((long long)(unsigned)__float_as_int(q.y) << 32) | (unsigned)__float_as_int(q.x));
 }
 
-// Symmetric blocks of the near field (Plan::sym_*): one CTA (4 warps) per
-// work item, or part of one (part of the sources of one chunk of <= 32
+// Symmetric blocks of the near field (Plan::sym_*) in FP64: one CTA (4 warps)
+// per work item, or part of one (part of the sources of one chunk of <= 32
 // targets), taken from a queue in the host's order of decreasing work; part p
 // of split takes every split-th round of 256 sources.  A lane owns S
 // sources and meets the chunk's targets in blocks of 4, read from shared
@@ -2443,38 +2439,32 @@ __device__ __forceinline__ double charge_word(float2 q) {
 // targets' sums around gave 76-86%; and 8 independent evaluations per lane
 // keep the FP64 pipe fed (65% of its cycles on a 31k-point sphere).  The near
 // field of a 250k-point sphere in FP64 took 20.1 ms with the segments and
-// takes 14.0 ms so; of a 600k-point sphere in mixed precision 22.5 and 20.3 ms.
-template <bool MIXED>
+// takes 14.1 ms so.
 struct P2PSym {
   static constexpr int S = 2;       // sources per lane
   static constexpr int NB = 8;      // blocks of 4 targets in a chunk
-  typedef typename std::conditional<MIXED, float4, double2>::type A;  // (sum, compensation) or sum
 };
 
-template <bool MIXED>
 __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, const int32_t* __restrict__ order,
                                                  const int32_t* __restrict__ item_chunk,
                                                  const int32_t* __restrict__ tfirst, const int32_t* __restrict__ tn,
                                                  const int64_t* __restrict__ ptr, const int32_t* __restrict__ sfirst,
                                                  const int32_t* __restrict__ sn, const int64_t* __restrict__ soff,
-                                                 const void* __restrict__ qv, double2* __restrict__ tpart,
-                                                 void* __restrict__ scratch, int split, unsigned long long* __restrict__ queue) {
-  typedef typename std::conditional<MIXED, float2, double2>::type Q;
-  typedef P2PSym<MIXED> G;
-  typedef typename G::A Acc;
+                                                 const double2* __restrict__ q, double2* __restrict__ tpart,
+                                                 double2* __restrict__ scr, int split, unsigned long long* __restrict__ queue) {
+  typedef double2 Q;
+  typedef P2PSym G;
   constexpr int RMAX = 128, S = G::S, NB = G::NB;
-  const Q* q = static_cast<const Q*>(qv);
-  Q* scr = static_cast<Q*>(scratch);
-  __shared__ double2 trxy[4 * NB], trzw[4 * NB];
-  __shared__ double2 tq[MIXED ? 1 : 4 * NB];  // FP64 path: target charges
-  __shared__ Acc tacc[4][NB][32];
+  __shared__ double2 trxy[4 * NB], tq[4 * NB];
+  __shared__ double trz[4 * NB];
+  __shared__ Q tacc[4][NB][32];
   __shared__ int32_t rpre[RMAX + 1], rfst[RMAX];
   __shared__ int64_t roff[RMAX];
   __shared__ double2 red[4][32];
   __shared__ int64_t cur;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double kq = P.kappa * 0.63661977236758134308;  // 2 k / pi
-  const double scale = MIXED ? 1. : 1. / (4. * 3.14159265358979323846);
+  const double scale = 1. / (4. * 3.14159265358979323846);
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
@@ -2489,17 +2479,11 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
     if (threadIdx.x < 4 * NB) {
       const int t = threadIdx.x;
       const double* x = P.T_pos + 3 * (int64_t)(f + (t < nt ? t : 0));
-      const Q qt = t < nt ? q[f + t] : Q{0, 0};
-      const double2 xy = make_double2(x[0], x[1]);
-      double2 zw = make_double2(x[2], 0.);
-      if constexpr (MIXED)
-        zw.y = charge_word(qt);
-      else
-        tq[t] = qt;
-      trxy[t] = xy;
-      trzw[t] = zw;
+      trxy[t] = make_double2(x[0], x[1]);
+      trz[t] = x[2];
+      tq[t] = t < nt ? q[f + t] : Q{0, 0};
     }
-    for (int b = 0; b < nb; b++) tacc[warp][b][lane] = Acc{};
+    for (int b = 0; b < nb; b++) tacc[warp][b][lane] = Q{0, 0};
     const int64_t rb = ptr[it], re = ptr[it + 1];
     for (int64_t r0 = rb; r0 < re; r0 += RMAX) {
       const int nr = (int)min((int64_t)RMAX, re - r0);
@@ -2559,11 +2543,12 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
           int least = INT_MAX;
 #pragma unroll
           for (int t = 0; t < 4; t++) {
-            const double2 a = trxy[4 * b + t], z = trzw[4 * b + t];
+            const double2 a = trxy[4 * b + t];
+            const double z = trz[4 * b + t];
             d[t] = Q{0, 0};
 #pragma unroll
             for (int v = 0; v < S; v++) {
-              const double dx = a.x - yx[v], dy = a.y - yy[v], dz = z.x - yz[v];
+              const double dx = a.x - yx[v], dy = a.y - yy[v], dz = z - yz[v];
               R[t][v] = fma(dx, dx, fma(dy, dy, dz * dz));
               least = min(least, __double2hiint(R[t][v]));
             }
@@ -2574,14 +2559,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
             for (int t = 0; t < 4; t++) {
 #pragma unroll
               for (int v = 0; v < S; v++) {
-                Q g, qi;
-                if constexpr (MIXED) {
-                  g = green32_r<GUARD>(R[t][v], P.kappa);
-                  qi = charge_bits(trzw[4 * b + t].y);
-                } else {
-                  g = green64_r<GUARD>(R[t][v], kq);
-                  qi = tq[4 * b + t];
-                }
+                const Q g = green64_r<GUARD>(R[t][v], kq), qi = tq[4 * b + t];
                 d[t].x = fma(g.x, qj[v].x, fma(-g.y, qj[v].y, d[t].x));
                 d[t].y = fma(g.x, qj[v].y, fma(g.y, qj[v].x, d[t].y));
                 accT[v].x = fma(g.x, qi.x, fma(-g.y, qi.y, accT[v].x));
@@ -2605,37 +2583,23 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
           s0 = h0 ? k0 : k1;
           kk.x += __shfl_xor_sync(0xffffffffu, s0.x, 8);
           kk.y += __shfl_xor_sync(0xffffffffu, s0.y, 8);
-          Acc o = tacc[warp][b][lane];
-          if constexpr (MIXED) {
-            kahan_add(o.x, o.y, kk.x);
-            kahan_add(o.z, o.w, kk.y);
-          } else {
-            o.x += kk.x;
-            o.y += kk.y;
-          }
+          Q o = tacc[warp][b][lane];
+          o.x += kk.x;
+          o.y += kk.y;
           tacc[warp][b][lane] = o;
         }
 #pragma unroll
         for (int v = 0; v < S; v++)
           if (sidx[v] >= 0) {
-            if constexpr (!MIXED) {
-              accT[v].x *= scale;
-              accT[v].y *= scale;
-            }
+            accT[v].x *= scale;
+            accT[v].y *= scale;
             scr[sidx[v]] = accT[v];
           }
       }
     }
     for (int b = 0; b < nb; b++) {
-      const Acc o = tacc[warp][b][lane];
-      double pr, pim;
-      if constexpr (MIXED) {
-        pr = (double)o.x - (double)o.y;
-        pim = (double)o.z - (double)o.w;
-      } else {
-        pr = o.x * scale;
-        pim = o.y * scale;
-      }
+      const Q o = tacc[warp][b][lane];
+      double pr = o.x * scale, pim = o.y * scale;
 #pragma unroll
       for (int w = 4; w; w >>= 1) {
         pr += __shfl_xor_sync(0xffffffffu, pr, w);
@@ -2651,6 +2615,159 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
         a.y += red[w][threadIdx.x].y;
       }
       tpart[(it * split + part) * 32 + threadIdx.x] = a;
+    }
+  }
+}
+
+// The same blocks in mixed precision: their FP32 sums keep one order, pair by
+// pair, so they go by segments.  tp steps of a block: lane ls owns one source
+// (y, qj) and meets target (ls + step) mod tp; the target's running sum moves
+// one lane down per step.  TP = 32 fixes the segment width at compile time.
+// Target records in shared memory as two 16-byte arrays, (x, y) and (z, w)
+// with w the charge's bits: one conflict-free 16-byte load from each per step.
+// Entry j holds target j mod tp (j < 64), so step st of lane ls reads entry
+// ls + st without wrapping arithmetic.
+template <int TP>
+__device__ __forceinline__ void sym_steps(int ls, int tp_rt, double yx, double yy, double yz, float2 qj,
+                                          const double2* trxy, const double2* trzw, double kappa, float2& accD,
+                                          float2& accT) {
+  const int tp = TP ? TP : tp_rt;
+  const double2* txy = trxy + ls;
+  const double2* tzw = trzw + ls;
+#pragma unroll 8
+  for (int st = 0; st < tp; st++) {
+    const double2 a = txy[st], b = tzw[st];
+    const float2 g = green32(a.x - yx, a.y - yy, b.x - yz, kappa);
+    const float2 qi = charge_bits(b.y);
+    accD.x = fmaf(g.x, qj.x, fmaf(-g.y, qj.y, accD.x));
+    accD.y = fmaf(g.x, qj.y, fmaf(g.y, qj.x, accD.y));
+    accT.x = fmaf(g.x, qi.x, fmaf(-g.y, qi.y, accT.x));
+    accT.y = fmaf(g.x, qi.y, fmaf(g.y, qi.x, accT.y));
+    accD.x = __shfl_sync(0xffffffffu, accD.x, ls + 1, tp);
+    accD.y = __shfl_sync(0xffffffffu, accD.y, ls + 1, tp);
+  }
+}
+
+// One CTA (4 warps) per work item; a warp splits into segments of tp =
+// nextpow2(nt) lanes; lane l of a segment owns source l of the segment's
+// tp-source sub-tile and, over tp steps, meets every target i = (l + step)
+// mod tp.  The target's partial is an accumulator that moves one lane down per
+// step and ends in lane i (compensated sums over the sub-tiles); the source's
+// is lane-local.  Issue bound: 64 instructions per evaluation, 76-86% of the
+// evaluated pairs count (600k-point sphere 22.5 ms; sources in lanes as above
+// take 19.6 ms, but round the FP32 sums differently by 2e-7).
+__global__ void __launch_bounds__(128) k_p2p_sym_mixed(DevPlan P, int64_t nwork, const int32_t* __restrict__ order,
+                                                 const int32_t* __restrict__ item_chunk,
+                                                 const int32_t* __restrict__ tfirst, const int32_t* __restrict__ tn,
+                                                 const int64_t* __restrict__ ptr, const int32_t* __restrict__ sfirst,
+                                                 const int32_t* __restrict__ sn, const int64_t* __restrict__ soff,
+                                                 const float2* __restrict__ q, double2* __restrict__ tpart,
+                                                 float2* __restrict__ scr, unsigned long long* __restrict__ queue) {
+  typedef float2 Q;
+  constexpr int RMAX = 128;
+  __shared__ double2 trxy[64], trzw[64];
+  __shared__ int32_t rpre[RMAX + 1], rfst[RMAX];
+  __shared__ int64_t roff[RMAX];
+  __shared__ double2 red[4][32];
+  __shared__ int64_t cur;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) cur = (int64_t)atomicAdd(queue, 1ULL);
+    __syncthreads();
+    const int64_t k = cur;
+    if (k >= nwork) break;
+    const int64_t it = order[k];
+    const int64_t ch = item_chunk[it];
+    const int f = tfirst[ch], nt = tn[ch];
+    int tp = 4;
+    while (tp < nt) tp <<= 1;
+    const int ls = lane & (tp - 1);
+    if (threadIdx.x < 64) {
+      const int j = threadIdx.x, t = j & (tp - 1);
+      if (t < nt) {
+        const double* x = P.T_pos + 3 * (int64_t)(f + t);
+        const Q qt = q[f + t];
+        trxy[j] = make_double2(x[0], x[1]);
+        trzw[j] = make_double2(x[2], charge_word(qt));
+      } else {
+        trxy[j] = make_double2(0., 0.);
+        trzw[j] = make_double2(0., 0.);
+      }
+    }
+    float sr = 0.f, cr = 0.f, si = 0.f, ci = 0.f;  // compensated target sums
+    const int64_t rb = ptr[it], re = ptr[it + 1];
+    for (int64_t r0 = rb; r0 < re; r0 += RMAX) {
+      const int nr = (int)min((int64_t)RMAX, re - r0);
+      __syncthreads();  // previous batch of ranges (and the target arrays) settled
+      for (int m = threadIdx.x; m < nr; m += blockDim.x) {
+        rfst[m] = sfirst[r0 + m];
+        roff[m] = soff[r0 + m];
+        rpre[m + 1] = sn[r0 + m];
+      }
+      __syncthreads();
+      if (warp == 0) {  // inclusive scan of the range lengths
+        int carry = 0;
+        for (int b0 = 0; b0 < nr; b0 += 32) {
+          int v = b0 + lane < nr ? rpre[b0 + lane + 1] : 0;
+          for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+          }
+          if (b0 + lane < nr) rpre[b0 + lane + 1] = carry + v;
+          carry += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) rpre[0] = 0;
+      }
+      __syncthreads();
+      const int ntot = rpre[nr];
+      for (int base = warp * 32; base < ntot; base += 4 * 32) {
+        const int jj = base + lane;
+        const bool vj = jj < ntot;
+        double yx = 0., yy = 0., yz = 0.;
+        Q qj = Q{0, 0};
+        int64_t sidx = 0;
+        if (vj) {
+          int lo = 0, hi = nr - 1;  // last range with rpre <= jj
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (rpre[mid] <= jj) lo = mid; else hi = mid - 1;
+          }
+          const int o = jj - rpre[lo];
+          const int64_t sj = (int64_t)rfst[lo] + o;
+          sidx = roff[lo] + o;
+          const double* y = P.S_pos + 3 * sj;
+          yx = y[0];
+          yy = y[1];
+          yz = y[2];
+          qj = q[sj];
+        }
+        Q accD = Q{0, 0}, accT = Q{0, 0};
+        // no validity tests: padded targets and missing sources carry zero
+        // charges, and their target sums are never stored
+        if (tp == 32)
+          sym_steps<32>(ls, 32, yx, yy, yz, qj, trxy, trzw, P.kappa, accD, accT);
+        else
+          sym_steps<0>(ls, tp, yx, yy, yz, qj, trxy, trzw, P.kappa, accD, accT);
+        kahan_add(sr, cr, accD.x);
+        kahan_add(si, ci, accD.y);
+        if (vj) scr[sidx] = accT;
+      }
+    }
+    double pr = (double)sr - (double)cr, pim = (double)si - (double)ci;
+    for (int o = tp; o < 32; o <<= 1) {  // segments of the warp hold the same targets
+      pr += __shfl_xor_sync(0xffffffffu, pr, o);
+      pim += __shfl_xor_sync(0xffffffffu, pim, o);
+    }
+    if (lane < tp) red[warp][lane] = make_double2(pr, pim);
+    __syncthreads();
+    if (threadIdx.x < nt) {
+      double2 a = red[0][threadIdx.x];
+      for (int w = 1; w < 4; w++) {
+        a.x += red[w][threadIdx.x].x;
+        a.y += red[w][threadIdx.x].y;
+      }
+      tpart[it * 32 + threadIdx.x] = a;
     }
   }
 }
@@ -3067,11 +3184,11 @@ void launch_p2p_sym(bool fp64, const DevPlan& dp, int64_t nwork, const int32_t* 
   cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   const int grid = (int)std::min<int64_t>(nwork * split, (int64_t)nsm * std::max(1, std::min(blocks_per_sm, 64)));
   if (fp64)
-    k_p2p_sym<false><<<grid, 128, 0, s>>>(dp, nwork, order, item_chunk, tfirst, tn, ptr, sfirst, sn, soff, q, tpart,
-                                          scratch, split, queue);
+    k_p2p_sym<<<grid, 128, 0, s>>>(dp, nwork, order, item_chunk, tfirst, tn, ptr, sfirst, sn, soff,
+                                   (const double2*)q, tpart, (double2*)scratch, split, queue);
   else
-    k_p2p_sym<true><<<grid, 128, 0, s>>>(dp, nwork, order, item_chunk, tfirst, tn, ptr, sfirst, sn, soff, q, tpart,
-                                         scratch, split, queue);
+    k_p2p_sym_mixed<<<grid, 128, 0, s>>>(dp, nwork, order, item_chunk, tfirst, tn, ptr, sfirst, sn, soff,
+                                         (const float2*)q, tpart, (float2*)scratch, queue);
 }
 
 void launch_p2p_reduce(bool fp64, int64_t nleaf, const int32_t* first, const int32_t* n, const int64_t* rptr,

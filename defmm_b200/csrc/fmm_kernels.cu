@@ -710,12 +710,13 @@ struct M2FCfg {
 // One line of the forward DFT: out(k) = sum_a v[a] w^(k a), k < P = 2 L - 1,
 // a < L.  Outputs k and P - k are A - i B and A + i B with A = sum cos v,
 // B = sum sin v: 4 (L - 1) FMAs for the two instead of 8 (L - 1) for each.
+// Order 7 goes term by term too (the paired sums spill: 6.3 and 5.7 ms).
 // FP32 sums go term by term: paired they take 9.3 instead of 11.1 ms (spheroid
 // 500k order 6) but round differently, and mixed results keep their bits.
 template <typename T, int L, typename C, typename Put>
 __device__ __forceinline__ void fdft_line(const C (&v)[L], Put put) {
   constexpr int P = 2 * L - 1;
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 4 || L >= 7) {
 #pragma unroll
     for (int k = 0; k < P; k++) {
       C o = v[0];
@@ -955,6 +956,8 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
 // current item's inverse DFTs run, so that an item starts with its spectra
 // loads instead of a chain of three misses (index, pointers, entries).
 // NL lists per item, for up to kCap entries each (the rest is read directly).
+// M2L with this and only the target slots that have a list: sphere 250k FP64
+// 43.8 -> 38.2 ms, 600k mixed 47.1 -> 43.9, eight right-hand sides 160 -> 128.
 template <int NL, int NT>
 struct M2LQueue {
   static constexpr int kCap = NT / NL < 64 ? NT / NL : 64;
@@ -1162,9 +1165,13 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_
 // spectra of its source slot, so the spectra traffic per right-hand side is
 // e P^3 (1 + 1/RB) per far pair instead of 2 e P^3.
 // CTAs per SM of k_m2l_rhs: room for K x RB complex accumulators per thread
-template <typename T, int NT, int RB>
+// (FP64 at order 7, K RB = 36: 768 threads per SM spill 2 KB per thread, M2L of
+// four right-hand sides on 30k points 47.8 ms, 512 threads 21.5 ms; with
+// K RB = 24, order 6, 768 are enough)
+template <typename T, int L, int NT, int RB>
 constexpr int m2l_rhs_ctas() {
-  return (sizeof(T) == 8 ? (RB >= 8 ? 512 : (RB >= 2 ? 768 : 1024)) : (RB >= 8 ? 768 : 1024)) / NT;
+  constexpr int K = ((2 * L - 1) * (2 * L - 1) * (2 * L - 1) + NT - 1) / NT;
+  return (sizeof(T) == 8 ? (RB >= 8 || K * RB > 24 ? 512 : (RB >= 2 ? 768 : 1024)) : (RB >= 8 ? 768 : 1024)) / NT;
 }
 // up to 4 right-hand sides per CTA whose spectra take at most 24 KB (FP32 at
 // orders <= 5, FP64 <= 4): the inverse DFTs of a target slot's RB spectra run
@@ -1175,7 +1182,7 @@ __host__ __device__ constexpr bool m2l_rhs_joint() {
 }
 
 template <typename T, int L, int NT, int RB>
-__global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, NT, RB>()) k_m2l_rhs(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1, int R,
+__global__ void __launch_bounds__(NT, m2l_rhs_ctas<T, L, NT, RB>()) k_m2l_rhs(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1, int R,
                                                              const typename cpx_t<T>::type* __restrict__ F,
                                                              const typename cpx_t<T>::type* __restrict__ ptab,
                                                              typename cpx_t<T>::type* __restrict__ Lx,
@@ -2980,7 +2987,7 @@ struct Launch {
                          const void* ptab, void* Lx, unsigned long long* queue, int nsm, cudaStream_t s) {
     constexpr int RBE = RB <= kMaxRB ? RB : 1;
     const int64_t nwork = (u1 - u0) * (R / RBE);
-    const int grid = (int)std::min<int64_t>(nwork, (int64_t)nsm * m2l_rhs_ctas<T, NT, RBE>());
+    const int grid = (int)std::min<int64_t>(nwork, (int64_t)nsm * m2l_rhs_ctas<T, L, NT, RBE>());
     k_m2l_rhs<T, L, NT, RBE><<<grid, NT, smem_m2l_rhs<RBE>(), s>>>(dp, u0, u1, f0, f1, R, (const C*)F, (const C*)ptab,
                                                           (C*)Lx, queue);
   }

@@ -536,3 +536,22 @@ def test_near_field_coincident_points_in_two_leaves(gap, counts, gpu):
     assert (abs(ref[10]) > 1e5) == counts
     A.set_precision("mixed")
     assert rel(A.matvec(q), ref) <= MIXED_TOL
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("apart", [False, True])
+def test_a_non_finite_charge_stays_out_of_its_own_potential(apart, value, gpu):
+    # pairs at distance 0 are skipped (P2P.hpp:66), whatever the charge: the
+    # potential at the point itself is that of the other charges
+    p = W.sphere_surface(2500, seed=41, wavelengths=4).points
+    trg = p[:2000] if apart else p  # distinct sets: the target-side near field alone
+    q = W.charges(len(p), 8)
+    A = make(p, trg, 4, 33, 2 * np.pi * 2)
+    for prec in ("fp64", "mixed"):
+        A.set_precision(prec)
+        for i in (0, 777, 1999):
+            z = q.copy()
+            z[i] = 0.0
+            without = A.matvec(z)[i]
+            z[i] = value
+            assert abs(A.matvec(z)[i] - without) <= 1e-12 * abs(without)

@@ -2,6 +2,7 @@
 // and interpolation order (L).  See kernels.cuh for the memory layout.
 #include "kernels.cuh"
 #include "device_math.cuh"
+#include "green64.cuh"
 #include "fmm_kernels.h"
 #include "ptx.cuh"
 
@@ -1920,63 +1921,6 @@ __global__ void __launch_bounds__(128, 3)
 // Source record in shared memory: a = (x, y), b = (z, charge) with the FP32
 // charge bits in b.y (mixed) or the FP64 charge in c (FP64 path).
 
-// Approximate FP64 reciprocal square root (the PTX instruction
-// rsqrt.approx.ftz.f64, about FP32 accuracy); callers refine it by Newton
-// steps y <- y (3/2 - R y^2 / 2), each of which doubles the correct bits.
-__device__ __forceinline__ double rsqrt_approx64(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return y;
-}
-
-// exp(i k r) / r of one pair in FP64 (0 for R < 1e-16, P2P.hpp:66), without
-// the factor 1 / (4 pi), with kq = 2 k / pi.  An FP64 instruction takes two
-// issue cycles, every other one, so both counts matter (41 FP64 instructions
-// here; the reduction by pi/2 in two parts with rint and Taylor series took
-// 48 and two conversions): 1/r from the approximate
-// reciprocal square root by one cubic step y + y e (1/2 + 3/8 e),
-// e = 1 - R y^2 (|e| < 2^-19: the next term is below 2^-58); the phase in
-// quarter turns, r kq = n + u with |u| <= 1/2, u by one exactly rounded FMA
-// and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
-// (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
-// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20).
-// GUARD = false: the caller knows R0 >= 1e-16.
-template <bool GUARD>
-__device__ __forceinline__ double2 green64_r(double R0, double kq) {
-  double R = R0;
-  if (GUARD) R = __hiloint2double(max(__double2hiint(R0), 0x3C9CD2B2), __double2loint(R0));
-  const double y0 = rsqrt_approx64(R);
-  const double e = fma(-(R * y0), y0, 1.0);
-  double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
-  const double r = R * y;
-  const double t = fma(r, kq, 6755399441055744.0);  // + 1.5 * 2^52
-  const double u = fma(r, kq, -(t - 6755399441055744.0));
-  const int q = __double2loint(t);
-  const double z = u * u;
-  double ps = fma(z, 5.633721016484235e-08, -3.598641754487236e-06);
-  ps = fma(z, ps, 0.00016044115029166428);
-  ps = fma(z, ps, -0.00468175413228242);
-  ps = fma(z, ps, 0.07969262624603957);
-  ps = fma(z, ps, -0.6459640975062443);
-  ps = fma(z, ps, 1.5707963267948966);
-  double pc = fma(z, -6.321892625650177e-09, 4.7106156592722383e-07);
-  pc = fma(z, pc, -2.5202036991591028e-05);
-  pc = fma(z, pc, 0.0009192602742250428);
-  pc = fma(z, pc, -0.020863480763315442);
-  pc = fma(z, pc, 0.2536695079010469);
-  pc = fma(z, pc, -1.2337005501361697);
-  pc = fma(z, pc, 1.0);
-  if (GUARD && __double_as_longlong(R0) < 0x3C9CD2B297D889BCLL) y = 0.;  // R0 < 1e-16
-  // quadrant q: sin and cos of the whole phase are (sr, cr), (cr, -sr),
-  // (-sr, -cr), (-cr, sr); both signs of q & 2 go into 1/r
-  const double K = __hiloint2double(__double2hiint(y) ^ (int)((unsigned)q << 30 & 0x80000000u), __double2loint(y));
-  const double sr = u * K * ps, cr = K * pc;
-  return make_double2((q & 1) ? -sr : cr, (q & 1) ? cr : sr);
-}
-__device__ __forceinline__ double2 green64(double dx, double dy, double dz, double kq) {
-  return green64_r<true>(fma(dx, dx, fma(dy, dy, dz * dz)), kq);
-}
-
 // Compensated (Kahan) FP32 summation: s - c carries the sum.
 __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
   const float y = x - c;
@@ -2553,7 +2497,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
           // the evaluations without a test of their own
           Q d[4];
           double R[4][S];
-          int least = INT_MAX;
+          unsigned least = UINT_MAX;
 #pragma unroll
           for (int t = 0; t < 4; t++) {
             const double2 a = trxy[4 * b + t];
@@ -2563,7 +2507,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
             for (int v = 0; v < S; v++) {
               const double dx = a.x - yx[v], dy = a.y - yy[v], dz = z - yz[v];
               R[t][v] = fma(dx, dx, fma(dy, dy, dz * dz));
-              least = min(least, __double2hiint(R[t][v]));
+              least = min(least, (unsigned)__double2hiint(R[t][v]));
             }
           }
           auto block = [&](auto guard) {
@@ -2580,7 +2524,7 @@ __global__ void __launch_bounds__(128, 4) k_p2p_sym(DevPlan P, int64_t nwork, co
               }
             }
           };
-          if (__any_sync(0xffffffffu, least <= 0x3C9CD2B2))
+          if (__any_sync(0xffffffffu, least <= kNearR2Hi))
             block(std::true_type());
           else
             block(std::false_type());

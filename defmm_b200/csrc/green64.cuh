@@ -14,8 +14,14 @@ __device__ __forceinline__ double rsqrt_approx64(double x) {
 }
 #endif
 
-constexpr unsigned long long kNearR2 = 0x3C9CD2B297D889BCull;  // the bits of 1e-16
-constexpr unsigned kNearR2Hi = 0x3C9CD2B2u;                    // and their high word
+// Squared distances below 1e-16 are coincident points' (P2P.hpp:66).  The bits
+// are compared as unsigned numbers: a squared distance is not negative, and a
+// NaN of either sign (a coordinate that is NaN) counts as a large one, so that
+// it reaches the potentials.
+constexpr unsigned kNearR2Hi = 0x3C9CD2B2u;  // the high word of 1e-16
+__device__ __forceinline__ bool coincident(double R) {
+  return (unsigned long long)__double_as_longlong(R) < 0x3C9CD2B297D889BCull;
+}
 
 // exp(i k r) / r of one pair in FP64 (0 for R < 1e-16, P2P.hpp:66), without
 // the factor 1 / (4 pi), with kq = 2 k / pi.  An FP64 instruction takes two
@@ -28,10 +34,7 @@ constexpr unsigned kNearR2Hi = 0x3C9CD2B2u;                    // and their high
 // and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
 // (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
 // Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20).
-// GUARD = false: the caller knows R0 >= 1e-16, or leaves the pair out itself.
-// The guard compares the bits as unsigned numbers: a squared distance is not
-// negative, and a NaN of either sign (a coordinate that is NaN) counts as a
-// large one, so that it reaches the potentials.
+// GUARD = false: the caller knows R0 >= 1e-16.
 template <bool GUARD>
 __device__ __forceinline__ double2 green64_r(double R0, double kq) {
   double R = R0;
@@ -57,7 +60,7 @@ __device__ __forceinline__ double2 green64_r(double R0, double kq) {
   pc = fma(z, pc, 0.2536695079010469);
   pc = fma(z, pc, -1.2337005501361697);
   pc = fma(z, pc, 1.0);
-  if (GUARD && (unsigned long long)__double_as_longlong(R0) < kNearR2) y = 0.;  // R0 < 1e-16
+  if (GUARD && coincident(R0)) y = 0.;
   // quadrant q: sin and cos of the whole phase are (sr, cr), (cr, -sr),
   // (-sr, -cr), (-cr, sr); both signs of q & 2 go into 1/r
   const double K = __hiloint2double(__double2hiint(y) ^ (int)((unsigned)q << 30 & 0x80000000u), __double2loint(y));

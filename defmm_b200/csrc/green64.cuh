@@ -23,6 +23,30 @@ __device__ __forceinline__ bool coincident(double R) {
   return (unsigned long long)__double_as_longlong(R) < 0x3C9CD2B297D889BCull;
 }
 
+// sin(pi/2 u) / u and cos(pi/2 u) for |u| <= 1/2, z = u^2: polynomials of degree
+// 6 and 7 in z, fitted with the Remez exchange in 50 digits and rounded to
+// doubles.  The rounding is what is left: with these coefficients the sine is
+// off by 5.0e-17 relative, the cosine by 1.6e-17 (an ulp is 1.1e-16 to 2.2e-16).
+template <class F>
+__device__ __forceinline__ F quarter_sin(F z) {
+  F p = fma(z, F(5.633721016484235e-08), F(-3.598641754487236e-06));
+  p = fma(z, p, F(0.00016044115029166428));
+  p = fma(z, p, F(-0.00468175413228242));
+  p = fma(z, p, F(0.07969262624603957));
+  p = fma(z, p, F(-0.6459640975062443));
+  return fma(z, p, F(1.5707963267948966));
+}
+template <class F>
+__device__ __forceinline__ F quarter_cos(F z) {
+  F p = fma(z, F(-6.321892625650177e-09), F(4.7106156592722383e-07));
+  p = fma(z, p, F(-2.5202036991591028e-05));
+  p = fma(z, p, F(0.0009192602742250428));
+  p = fma(z, p, F(-0.020863480763315442));
+  p = fma(z, p, F(0.2536695079010469));
+  p = fma(z, p, F(-1.2337005501361697));
+  return fma(z, p, F(1.0));
+}
+
 // exp(i k r) / r of one pair in FP64 (0 for R < 1e-16, P2P.hpp:66), without
 // the factor 1 / (4 pi), with kq = 2 k / pi.  An FP64 instruction takes two
 // issue cycles, every other one, so both counts matter (41 FP64 instructions
@@ -31,9 +55,11 @@ __device__ __forceinline__ bool coincident(double R) {
 // reciprocal square root by one cubic step y + y e (1/2 + 3/8 e),
 // e = 1 - R y^2 (|e| < 2^-19: the next term is below 2^-58); the phase in
 // quarter turns, r kq = n + u with |u| <= 1/2, u by one exactly rounded FMA
-// and n's low bits from the mantissa of r kq + 1.5 * 2^52; sin(pi/2 u) / u and
-// (cos(pi/2 u) - 1) / u^2 by polynomials of degree 6 in u^2, fitted with the
-// Remez exchange in 50 digits (errors below 4e-18 relative and 4e-20).
+// and n's low bits from the mantissa of r kq + 1.5 * 2^52.  kq is rounded once,
+// so all pairs share its relative error (up to 1.1e-16): at k r near 35 the
+// phase's mean error can reach a few 1e-15, as much as its scatter (3.6e-15
+// rms, from rounding r); reducing by pi/2 in two parts shares less (3e-16)
+// with the same scatter and larger maxima.
 // GUARD = false: the caller knows R0 >= 1e-16.
 template <bool GUARD>
 __device__ __forceinline__ double2 green64_r(double R0, double kq) {
@@ -47,19 +73,7 @@ __device__ __forceinline__ double2 green64_r(double R0, double kq) {
   const double u = fma(r, kq, -(t - 6755399441055744.0));
   const int q = __double2loint(t);
   const double z = u * u;
-  double ps = fma(z, 5.633721016484235e-08, -3.598641754487236e-06);
-  ps = fma(z, ps, 0.00016044115029166428);
-  ps = fma(z, ps, -0.00468175413228242);
-  ps = fma(z, ps, 0.07969262624603957);
-  ps = fma(z, ps, -0.6459640975062443);
-  ps = fma(z, ps, 1.5707963267948966);
-  double pc = fma(z, -6.321892625650177e-09, 4.7106156592722383e-07);
-  pc = fma(z, pc, -2.5202036991591028e-05);
-  pc = fma(z, pc, 0.0009192602742250428);
-  pc = fma(z, pc, -0.020863480763315442);
-  pc = fma(z, pc, 0.2536695079010469);
-  pc = fma(z, pc, -1.2337005501361697);
-  pc = fma(z, pc, 1.0);
+  const double ps = quarter_sin(z), pc = quarter_cos(z);
   if (GUARD && coincident(R0)) y = 0.;
   // quadrant q: sin and cos of the whole phase are (sr, cr), (cr, -sr),
   // (-sr, -cr), (-cr, sr); both signs of q & 2 go into 1/r

@@ -31,6 +31,7 @@ static int __double2loint(double x) { return (int)bits(x); }
 static long long __double_as_longlong(double x) { return (long long)bits(x); }
 static double __hiloint2double(int hi, int lo) { return from_bits((uint64_t)(uint32_t)hi << 32 | (uint32_t)lo); }
 using std::fma;
+static __float128 fma(__float128 a, __float128 b, __float128 c) { return fmaq(a, b, c); }
 using std::max;
 // an estimate off by up to 2^-20, to either side
 static double rsqrt_approx64(double x) { return 1. / std::sqrt(x) * (1. + ((bits(x) & 1) ? 9e-7 : -9e-7)); }
@@ -59,6 +60,20 @@ int main() {
     const double R = std::pow(10., -15.9 + 20. * U(rng)), kq = 100. * U(rng);
     const double2 a = green64_r<true>(R, kq), b = green64_r<false>(R, kq);
     assert(a.x == b.x && a.y == b.y);
+  }
+  // the rounded coefficients, evaluated in quad precision, against sin and cos:
+  // half an ulp of the leading ones (1.1e-16 of 1.57, the sine's) bounds what
+  // rounding can do, the stated 5.0e-17 and 1.6e-17 what it did
+  __float128 es = 0, ec = 0;
+  for (int i = 1; i <= 20000; i++) {
+    const __float128 u = (__float128)i / 40000, z = u * u;
+    const __float128 s = sinq(M_PI_2q * u), c = cosq(M_PI_2q * u);
+    es = std::max(es, fabsq(u * dfb::quarter_sin(z) / s - 1));
+    ec = std::max(ec, fabsq(dfb::quarter_cos(z) - c));
+  }
+  if (es > 5.05e-17Q || ec > 1.65e-17Q) {
+    std::printf("sine %.3g, cosine %.3g\n", (double)es, (double)ec);
+    return 1;
   }
   std::puts("ok");
   return 0;

@@ -2380,10 +2380,15 @@ __device__ __forceinline__ double charge_word(float2 q) {
 
 // Symmetric blocks of the near field (Plan::sym_*) in FP64: one CTA (4 warps)
 // per work item, or part of one (part of the sources of one chunk of <= 32
-// targets), taken from a queue in the host's order of decreasing work; part p
-// of split takes every split-th round of 256 sources.  A lane owns S
-// sources and meets the chunk's targets in blocks of 4, read from shared
-// memory by broadcast.  One evaluation of G feeds both
+// targets), taken from a queue in the host's order of decreasing work; of each
+// batch of up to 128 ranges, part p of split takes round p of 256 sources and
+// every split-th one after it.  (With tiny leaves a batch can have fewer rounds
+// than the item has parts; the other parts then only write zeros.  Counting on
+// over the batches evens that out but costs more than it gives: 20,000 points
+// in leaves of 4, up to 288 ranges per item, 1.94 and 1.95 ms; cube 20k 743 and
+// 745 us per matvec.)  A lane owns S sources and meets the chunk's targets in
+// blocks of 4, read from shared memory by broadcast.  One evaluation of G feeds
+// both
 //   the target's partial: 4 sums per block, over the lane's S sources; two
 //     exchange steps leave one target per lane (summed over 4 lanes), added
 //     to the lane's sum for this block in shared memory, and

@@ -555,3 +555,16 @@ def test_a_non_finite_charge_stays_out_of_its_own_potential(apart, value, gpu):
             without = A.matvec(z)[i]
             z[i] = value
             assert abs(A.matvec(z)[i] - without) <= 1e-12 * abs(without)
+
+
+def test_near_field_parts_of_items_with_many_ranges(gpu):
+    # a volume of tiny leaves inside a coarse surface: a chunk meets up to 288
+    # separate source ranges (more than a CTA holds at a time), in two parts
+    rng = np.random.default_rng(0)
+    p = np.vstack([W.sphere_surface(1000, seed=1).points, 0.3 + 0.3 * rng.normal(size=(4000, 3))])
+    q = W.charges(len(p), 8)
+    A = make(p, p, 4, 4, 60.0)
+    ref = A.matvec(q)
+    assert rel(ref, O.OracleFMM(p, p, 4, 4, 60.0, -1).gemv(q)) <= FP64_TOL
+    A.set_precision("mixed")
+    assert rel(A.matvec(q), ref) <= MIXED_TOL

@@ -1165,14 +1165,29 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_
 // transfer spectrum entry U_k[i] is loaded once and multiplied into the RB
 // spectra of its source slot, so the spectra traffic per right-hand side is
 // e P^3 (1 + 1/RB) per far pair instead of 2 e P^3.
-// CTAs per SM of k_m2l_rhs: room for K x RB complex accumulators per thread
-// (FP64 at order 7, K RB = 36: 768 threads per SM spill 2 KB per thread, M2L of
-// four right-hand sides on 30k points 47.8 ms, 512 threads 21.5 ms; with
-// K RB = 24, order 6, 768 are enough)
+// CTAs per SM of k_m2l_rhs, by the registers that its accumulators take
+// (A = K RB values of 2 or 4): more CTAs hide more latency until the registers
+// left for loads in flight run out.  Of 512, 768 and 1024 threads per SM this
+// takes the fastest (M2L, 30,001-point sphere, ms; blocks of 3, 4 or 8
+// right-hand sides):
+//   128 threads, A <= 22: order 4 FP64 RB = 1 (A = 12) 2.75 / 2.04 / 1.77
+//   128 threads, A 24-36: order 5 FP64 RB = 1 (24) 3.64 / 3.37 / 4.77, order 7
+//     FP32 RB = 1 (36) 5.79 / 5.42 / 6.31
+//   128 threads, A >= 44: order 6 FP64 RB = 1 (44) 6.05 / 7.17 / 8.96, order 6
+//     FP32 RB = 2 (44) 7.79 / 8.66 / 13.6, order 8 FP32 RB = 1 (54) 8.51 / 11.8 /
+//     16.6; order 7 FP64 RB = 2 (144, more than 128 registers hold) 21.3 / 48 /
+//     55 for four right-hand sides, 12.4 at 256
+//   256 threads: order 2 FP64 RB = 4 (16, K = 1) 1.63 / 1.12 / 0.85, order 5
+//     FP64 RB = 4 (48) 5.22 / 4.42 / 4.78, order 5 FP32 RB = 4 (24) 3.63 / 2.62 /
+//     2.12 and RB = 8 (48) 7.31 / 6.92 / 6.26, order 6 FP64 RB = 4 (96) 9.15 /
+//     12.3 / 14.5
 template <typename T, int L, int NT, int RB>
 constexpr int m2l_rhs_ctas() {
-  constexpr int K = ((2 * L - 1) * (2 * L - 1) * (2 * L - 1) + NT - 1) / NT;
-  return (sizeof(T) == 8 ? (RB >= 8 || K * RB > 24 ? 512 : (RB >= 2 ? 768 : 1024)) : (RB >= 8 ? 768 : 1024)) / NT;
+  constexpr int P = 2 * L - 1, K = (P * P * P + NT - 1) / NT, A = K * RB * 2 * (int)sizeof(T) / 4;
+  constexpr int threads = NT == 128 ? (A <= 22 ? 1024 : A <= 36 ? 768 : A <= 112 ? 512 : 256)
+                                    : (A > 48 ? 512 : sizeof(T) == 4 || K == 1 ? 1024 : 768);
+  static_assert(A + 16 <= 65536 / threads, "the accumulators alone would spill");
+  return threads / NT;
 }
 // up to 4 right-hand sides per CTA whose spectra take at most 24 KB (FP32 at
 // orders <= 5, FP64 <= 4): the inverse DFTs of a target slot's RB spectra run

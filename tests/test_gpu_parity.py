@@ -568,3 +568,22 @@ def test_near_field_parts_of_items_with_many_ranges(gpu):
     assert rel(ref, O.OracleFMM(p, p, 4, 4, 60.0, -1).gemv(q)) <= FP64_TOL
     A.set_precision("mixed")
     assert rel(A.matvec(q), ref) <= MIXED_TOL
+
+
+@pytest.mark.parametrize("order", [5, 6, 7, 8])
+def test_blocks_at_high_orders(order, gpu):
+    # one, two and four right-hand sides per M2L CTA (as far as the order
+    # allows), whose accumulators take 24 to 144 registers
+    w = W.sphere_surface(5000, seed=21, wavelengths=5.0)
+    Q = np.stack([W.charges(w.n, 40 + r) for r in range(4)])
+    A = make(w.points, w.points, order, 64, w.kappa)
+    ref = O.OracleFMM(w.points, w.points, order, 64, w.kappa, -1).gemv(Q[1])
+    for prec, tol in (("fp64", FP64_TOL), ("mixed", MIXED_TOL)):
+        A.set_precision(prec)
+        A.set_blocking(1, 1)
+        one = A.matvec(Q[1])
+        assert rel(one, ref) <= tol
+        for R in (2, 3, 4):
+            A.set_blocking(R, 1)
+            P = A.matvec(Q[:R])
+            assert np.array_equal(P[1], one)

@@ -951,14 +951,18 @@ __device__ __forceinline__ void m2l_f2l(const typename cpx_t<T>::type* acc, type
   }
 }
 
-// Work queue of the M2L kernels: CTAs take work items in order (so the target
-// slots in flight stay a contiguous window of one cone, and F_s and U_k are
-// served from L2) and fetch the next item's index and lists while the
-// current item's inverse DFTs run, so that an item starts with its spectra
-// loads instead of a chain of three misses (index, pointers, entries).
-// NL lists per item, for up to kCap entries each (the rest is read directly).
-// M2L with this and only the target slots that have a list: sphere 250k FP64
-// 43.8 -> 38.2 ms, 600k mixed 47.1 -> 43.9, eight right-hand sides 160 -> 128.
+// Work queue of k_m2l and k_m2l_rhs.  A CTA's first item is its own number, the
+// others come from the queue in order, so that the target slots in flight stay
+// a window of one cone (F_s and U_k are served from L2); of the CTAs that do
+// not fit on the chip at first, the first items run late and outside that
+// window.  The next item's index and list are fetched while the current item's
+// inverse DFTs run, so that an item starts with its spectra loads instead of a
+// chain of three misses (index, pointers, entries): NL lists per item, up to
+// kCap entries each, the rest is read directly.  M2L with this and only the
+// target slots that have a list: sphere 250k FP64 43.8 -> 38.2 ms, 600k mixed
+// 47.1 -> 43.9, eight right-hand sides 160 -> 128.  (Both users have one list.
+// Without the list index the compiler orders the spectra loads differently and
+// the 250k sphere takes 41.8 ms, the 600k one 46.1.)
 template <int NL, int NT>
 struct M2LQueue {
   static constexpr int kCap = NT / NL < 64 ? NT / NL : 64;
@@ -1074,7 +1078,13 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(
 // source slot, so a merge of the two lists finds their common sources
 // (about a third of the pairs at order 5), whose spectrum F_s is then read
 // once for both.  Every accumulator sees its own list in list order with the
-// same operations as k_m2l, so the results are bit-identical to it.
+// same operations as k_m2l, so the results are bit-identical to it.  Both lists
+// are read from memory as the merge goes on and items all come from the queue:
+// M2LQueue for two lists took registers that the second accumulator set needs
+// and was the slower one (M2L, ms: sphere 250k FP64 39.7 and 38.5, 600k mixed
+// 48.2 and 44.0, 60k mixed order 6 8.6 and 7.0; 30,001 points order 4 FP64 at
+// 256 threads 1.74 and 1.19; only order 7 mixed at 256 threads the other way,
+// 2.22 and 2.43, where one slot per CTA takes 1.84).
 template <typename T, int L, int NT>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_pair(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
                                                             const typename cpx_t<T>::type* __restrict__ F,
@@ -1082,80 +1092,70 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_
                                                             typename cpx_t<T>::type* __restrict__ Lx,
                                                             unsigned long long* __restrict__ queue) {
   typedef typename cpx_t<T>::type C;
-  typedef M2LQueue<2, NT> Q;
   constexpr int PD = 2 * L - 1, LL = L * L * L, PP = PD * PD * PD, K = (PP + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Js = reinterpret_cast<C*>(smem_raw);
-  __shared__ typename Q::Shared qs;
-  const int64_t nwork = (u1 - u0 + 1) / 2;
-  Q q(qs, P, queue, nwork);
-  q.first(u0 + 2 * (int64_t)blockIdx.x, u1);
-  __syncthreads();
-  for (int ph = 0; qs.item[ph] < nwork; ph ^= 1) {
-    q.fetch();
-    const int64_t u = u0 + 2 * qs.item[ph];
+  __shared__ int64_t cur;
+  for (;;) {
+    __syncthreads();  // the previous slots' inverse DFTs are done with Js
+    if (threadIdx.x == 0) cur = u0 + 2 * (int64_t)atomicAdd(queue, 1ULL);
+    __syncthreads();
+    const int64_t u = cur;
+    if (u >= u1) break;
     const bool two = u + 1 < u1;
-    const int64_t t = P.m2l_tlist[u], t2 = P.m2l_tlist[two ? u + 1 : u];
-    const int ae = qs.len[ph][0], be = qs.len[ph][1];
+    int64_t a = P.m2l_cptr[u], b = P.m2l_cptr[u + 1];
+    const int64_t ae = b, be = two ? P.m2l_cptr[u + 2] : b;
     C acc0[K], acc1[K];
 #pragma unroll
     for (int k = 0; k < K; k++) acc0[k] = acc1[k] = czero<C>();
-    const int2 none = make_int2(INT_MAX, 0);
-    // the merge over entries at(list, x)
-    auto merge = [&](auto at) {
-      int a = 0, b = 0;
-      int2 ea = a < ae ? at(0, a) : none, eb = b < be ? at(1, b) : none;
-      while (a < ae || b < be) {
-        const int src = ea.x < eb.x ? ea.x : eb.x;
-        const bool ha = ea.x == src, hb = eb.x == src;
-        const int ka = ea.y, kb = eb.y;
-        if (ha) ea = ++a < ae ? at(0, a) : none;
-        if (hb) eb = ++b < be ? at(1, b) : none;
-        if (src < f0 || src >= f1) {  // entry outside this cone batch: a plan bug
-          if (threadIdx.x == 0) atomicExch(P.err, 1);
-          continue;
-        }
-        const C* Fs = F + (src - f0) * PP;
-        const C* U0 = ptab + (int64_t)(uint32_t)ka * PP;
-        const C* U1 = ptab + (int64_t)(uint32_t)kb * PP;
-        if (ha && hb) {
-#pragma unroll
-          for (int k = 0; k < K; k++) {
-            const int i = threadIdx.x + k * NT;
-            if (i < PP) {
-              const C f = __ldg(Fs + i);
-              cfma(acc0[k], __ldg(U0 + i), f);
-              cfma(acc1[k], __ldg(U1 + i), f);
-            }
-          }
-        } else if (ha) {
-#pragma unroll
-          for (int k = 0; k < K; k++) {
-            const int i = threadIdx.x + k * NT;
-            if (i < PP) cfma(acc0[k], __ldg(U0 + i), __ldg(Fs + i));
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < K; k++) {
-            const int i = threadIdx.x + k * NT;
-            if (i < PP) cfma(acc1[k], __ldg(U1 + i), __ldg(Fs + i));
-          }
-        }
+    while (a < ae || b < be) {
+      const int sa = a < ae ? P.m2l_src[a] : INT_MAX;
+      const int sb = b < be ? P.m2l_src[b] : INT_MAX;
+      const int src = sa < sb ? sa : sb;
+      if (src < f0 || src >= f1) {  // entry outside this cone batch: a plan bug
+        if (threadIdx.x == 0) atomicExch(P.err, 1);
+        if (sa == src) a++;
+        if (sb == src) b++;
+        continue;
       }
-    };
-    if (ae <= Q::kCap && be <= Q::kCap)
-      merge([&](int jj, int x) { return qs.e[ph][jj][x]; });
-    else
-      merge([&](int jj, int x) { return x < Q::kCap ? qs.e[ph][jj][x] : q.direct(ph, jj, x); });
-    q.publish(ph ^ 1);
-    m2l_f2l<T, L, NT, 1>(acc0, Js, [&](int) { return Lx + t * LL; }, [&] { q.pointers(qs.item[ph ^ 1], u0 + 2 * qs.item[ph ^ 1], u1); },
-                         [&] { q.entries(); });
+      const C* Fs = F + (src - f0) * PP;
+      if (sa == sb) {
+        const C* U0 = ptab + (int64_t)P.m2l_tab[a] * PP;
+        const C* U1 = ptab + (int64_t)P.m2l_tab[b] * PP;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          const int i = threadIdx.x + k * NT;
+          if (i < PP) {
+            const C f = __ldg(Fs + i);
+            cfma(acc0[k], __ldg(U0 + i), f);
+            cfma(acc1[k], __ldg(U1 + i), f);
+          }
+        }
+        a++;
+        b++;
+      } else if (sa < sb) {
+        const C* U0 = ptab + (int64_t)P.m2l_tab[a] * PP;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          const int i = threadIdx.x + k * NT;
+          if (i < PP) cfma(acc0[k], __ldg(U0 + i), __ldg(Fs + i));
+        }
+        a++;
+      } else {
+        const C* U1 = ptab + (int64_t)P.m2l_tab[b] * PP;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          const int i = threadIdx.x + k * NT;
+          if (i < PP) cfma(acc1[k], __ldg(U1 + i), __ldg(Fs + i));
+        }
+        b++;
+      }
+    }
+    m2l_f2l<T, L, NT, 1>(acc0, Js, [&](int) { return Lx + (int64_t)P.m2l_tlist[u] * LL; }, [] {}, [] {});
     if (two) {
       __syncthreads();
-      m2l_f2l<T, L, NT, 1>(acc1, Js, [&](int) { return Lx + t2 * LL; }, [] {}, [] {});
+      m2l_f2l<T, L, NT, 1>(acc1, Js, [&](int) { return Lx + (int64_t)P.m2l_tlist[u + 1] * LL; }, [] {}, [] {});
     }
-    q.store(ph ^ 1);
-    __syncthreads();
   }
 }
 

@@ -1023,12 +1023,25 @@ struct M2LQueue {
   }
 };
 
+// CTAs per SM of k_m2l (SLOTS = 1) and k_m2l_pair (2): 512 threads in FP64 and
+// 1,024 in FP32, but fewer where the accumulators (A registers) would spill and
+// more where there is one value per thread and 256 of them (M2L, 30,001-point
+// sphere, ms, without and with the exceptions): order 8 FP32 at 128 threads
+// (A = 54) 5.99 and 2.86, pairs at 128 threads order 8 FP32 (108) 8.70 and 5.10,
+// FP64 (216) 15.7 and 12.6, order 7 FP32 (72) 2.85 and 2.12, FP64 (144) 6.06 and
+// 4.03; orders 2 and 3 FP64 at 256 threads 0.71 and 0.54, 1.03 and 0.59.
+template <typename T, int L, int NT, int SLOTS>
+constexpr int m2l_ctas() {
+  constexpr int P = 2 * L - 1, K = (P * P * P + NT - 1) / NT, A = K * SLOTS * 2 * (int)sizeof(T) / 4;
+  return (A > 112 ? 256 : sizeof(T) == 8 ? (NT == 256 && K == 1 ? 1536 : 512) : A > 48 ? 512 : 1024) / NT;
+}
+
 // One CTA per listed target slot [u0, u1) of a cone batch (M2L.hpp:115-157
 // target-stationary, then the inverse DFT above):
 //   J[i] = sum_{(s, k) in list(t)} U_k[i] F_s[i]          (registers)
 // J never leaves the SM.
 template <typename T, int L, int NT>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
+__global__ void __launch_bounds__(NT, m2l_ctas<T, L, NT, 1>()) k_m2l(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
                                                        const typename cpx_t<T>::type* __restrict__ F,
                                                        const typename cpx_t<T>::type* __restrict__ ptab,
                                                        typename cpx_t<T>::type* __restrict__ Lx,
@@ -1086,7 +1099,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l(
 // 256 threads 1.74 and 1.19; only order 7 mixed at 256 threads the other way,
 // 2.22 and 2.43, where one slot per CTA takes 1.84).
 template <typename T, int L, int NT>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 512 : 1024) / NT) k_m2l_pair(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
+__global__ void __launch_bounds__(NT, m2l_ctas<T, L, NT, 2>()) k_m2l_pair(DevPlan P, int64_t u0, int64_t u1, int64_t f0, int64_t f1,
                                                             const typename cpx_t<T>::type* __restrict__ F,
                                                             const typename cpx_t<T>::type* __restrict__ ptab,
                                                             typename cpx_t<T>::type* __restrict__ Lx,

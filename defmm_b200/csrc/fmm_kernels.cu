@@ -756,7 +756,7 @@ __device__ __forceinline__ void fdft_line(const C (&v)[L], Put put) {
 }
 
 template <typename T, int L>
-__global__ void __launch_bounds__(256) k_m2f(int64_t n, int R, const int32_t* __restrict__ slist,
+__global__ void __launch_bounds__(256) k_m2f(int64_t nexp, int R, const int32_t* __restrict__ slist,
                                              const typename cpx_t<T>::type* __restrict__ M,
                                              typename cpx_t<T>::type* __restrict__ F) {
   typedef typename cpx_t<T>::type C;
@@ -770,32 +770,64 @@ __global__ void __launch_bounds__(256) k_m2f(int64_t n, int R, const int32_t* __
   // the next expansion is loaded into registers while the current one is
   // transformed
   constexpr int NV = (LL + 31) / 32;
-  const int64_t e0 = (int64_t)blockIdx.x * NW + warp, de = (int64_t)gridDim.x * NW;
+  // Expansion e is right-hand side r = e mod R of the (i = e / R)-th listed slot.
+  // Orders 4 to 6 wait for memory and divide; below and above, i and r go on
+  // without a division and the slot's number is read one round ahead of its
+  // values (eight right-hand sides, 30,001 points, dividing and not: mixed order
+  // 2 0.148 and 0.113 ms, 3 0.231 and 0.210, 7 4.91 and 3.98, 8 8.25 and 7.08,
+  // FP64 order 8 15.4 and 14.2; order 5 FP64 2.16 and 2.20).  There counts take
+  // 32 bits (the F buffer holds at most 64 GB of spectra), but not in FP32
+  // above order 6, where 64-bit ones make the compiler keep more loads in
+  // flight (order 7 4.76 and 3.98, order 8 8.02 and 7.08).
+  constexpr bool STEP = L < 4 || L > 6;
+  typedef typename std::conditional<STEP && (sizeof(T) == 8 || L < 4), int, int64_t>::type E;
+  const E n = (E)nexp, e0 = (E)blockIdx.x * NW + warp, de = (E)gridDim.x * NW;
+  int i = 0, r = 0, di = 0, dr = 0;
+  int32_t slot = 0;
+  if constexpr (STEP) {
+    i = (int)((unsigned)e0 / (unsigned)R), r = (int)((unsigned)e0 % (unsigned)R);
+    di = (int)((unsigned)de / (unsigned)R), dr = (int)((unsigned)de % (unsigned)R);
+    if (e0 < n) slot = slist[i];
+  }
+  // e: e0 first, then each next one
+  auto row = [&](E e) {
+    if constexpr (STEP) {
+      const C* Me = M + ((int64_t)slot * R + r) * LL;
+      i += di;
+      r += dr;
+      if (r >= R) {
+        r -= R;
+        i++;
+      }
+      if (e + de < n) slot = slist[i];
+      return Me;
+    } else {
+      return M + ((int64_t)slist[e / R] * R + e % R) * LL;
+    }
+  };
   C nx[NV];
-  // expansion e: right-hand side e mod R of the (e / R)-th listed slot
-  auto row = [&](int64_t e) { return M + ((int64_t)slist[e / R] * R + e % R) * LL; };
   if (e0 < n) {
     const C* Me = row(e0);
 #pragma unroll
     for (int m = 0; m < NV; m++) {
-      const int i = lane + 32 * m;
-      nx[m] = i < LL ? Me[i] : czero<C>();
+      const int j = lane + 32 * m;
+      nx[m] = j < LL ? Me[j] : czero<C>();
     }
   }
-  for (int64_t e = e0; e < n; e += de) {
+  for (E e = e0; e < n; e += de) {
     __syncwarp();
 #pragma unroll
     for (int m = 0; m < NV; m++) {
-      const int i = lane + 32 * m;
-      if (i < LL) Mi[i] = nx[m];
+      const int j = lane + 32 * m;
+      if (j < LL) Mi[j] = nx[m];
     }
     __syncwarp();
     if (e + de < n) {
       const C* Me = row(e + de);
 #pragma unroll
       for (int m = 0; m < NV; m++) {
-        const int i = lane + 32 * m;
-        if (i < LL) nx[m] = Me[i];
+        const int j = lane + 32 * m;
+        if (j < LL) nx[m] = Me[j];
       }
     }
     for (int ln = lane; ln < L * L; ln += 32) {  // axis 2: (a,b) lines
@@ -817,7 +849,7 @@ __global__ void __launch_bounds__(256) k_m2f(int64_t n, int R, const int32_t* __
       C v[L];
 #pragma unroll
       for (int a = 0; a < L; a++) v[a] = B[a * P * P + ln];
-      fdft_line<T, L>(v, [&](int k0, C o) { F[e * PP + k0 * P * P + ln] = o; });
+      fdft_line<T, L>(v, [&](int k0, C o) { F[(int64_t)e * PP + k0 * P * P + ln] = o; });
     }
   }
 }

@@ -69,7 +69,7 @@ struct defmm_handle {
   cudaStream_t st = nullptr, st2 = nullptr;  // own stream; near field
   cudaStream_t cur = nullptr;                // stream of the gemv in progress (phase events)
   std::vector<void*> plan_allocs;  // freed when the plan is rebuilt, like the slab's arrays
-  dfb::DeviceSlab plan_slab;
+  dfb::DeviceSlab plan_slab;       // (those that prcmpt leaves on the device, too)
   DevPlan dp;
   const dfb::OpTable* ops = nullptr;
   int ops_prec = -1;
@@ -577,7 +577,7 @@ int prepare_tables(defmm_handle* h) {
       return st;
     }
     std::string e;
-    st = dfb::device_plan_tables(p, (double2*)t64.p, (double2*)a64.p, (double2*)b64.p, e);
+    st = dfb::device_plan_tables(p, (double2*)t64.p, (double2*)a64.p, (double2*)b64.p, h->plan_slab, e);
     if (st) {
       free_buf(t64);
       free_buf(a64);
@@ -1665,6 +1665,7 @@ int defmm_prcmpt(defmm_handle* h, int L, int Ncrit, double kappa, int lvMAX) {
   h->built = false;
   h->uploaded = false;
   h->plan = Plan();
+  h->plan.dev_slab = &h->plan_slab;
   h->m2l_ranked = false;
   h->plan.keep_lists = h->keep_lists;
   std::string e;
@@ -1685,10 +1686,6 @@ int defmm_prcmpt(defmm_handle* h, int L, int Ncrit, double kappa, int lvMAX) {
   }
   int st = dfb::build_plan(h->plan, h->src.data(), (int64_t)h->src.size() / 3, h->trg.data(),
                            (int64_t)h->trg.size() / 3, L, Ncrit, kappa, lvMAX, e, walker, sorter.get());
-  // arrays the walk left on the device belong to this handle's plan (also
-  // when the build failed part way)
-  h->plan_allocs.insert(h->plan_allocs.end(), h->plan.dev_allocs.begin(), h->plan.dev_allocs.end());
-  h->plan.dev_allocs.clear();
   if (st) return h->fail(st == -4 ? DEFMM_ERR_CUDA : st == -5 ? DEFMM_ERR_MEMORY : st, e);
   h->walked_on_device = walker != nullptr;
   if (h->plan.lv.nlvl > 32) return h->fail(DEFMM_ERR_DEPTH, "more than 32 tree levels");

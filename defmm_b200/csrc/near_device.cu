@@ -344,21 +344,36 @@ __global__ void k_split_fill(int64_t nch, const int64_t* __restrict__ ptr, const
 
 #undef GRID_LOOP
 
-// Device memory of one build: scratch freed at the end, outputs handed to
-// the plan on success (freed here on failure).
+// Device memory of one build: scratch goes back at the end, outputs stay with
+// the plan on success (and go back on failure).
 struct Mem {
-  DeviceSlab tmp, out;
+  DeviceSlab &tmp, &out;
+  std::vector<void*> scratch, outputs;
   void* cub = nullptr;
   size_t cub_bytes = 0;
+  bool keep_outputs = false;
+  Mem(DeviceSlab& t, DeviceSlab& o) : tmp(t), out(o) {}
+  ~Mem() {
+    for (void* q : scratch) tmp.drop(q);
+    if (!keep_outputs)
+      for (void* q : outputs) out.drop(q);
+  }
   template <class T>
   T* get(int64_t n, bool keep = false) {
-    return static_cast<T*>((keep ? out : tmp).get((size_t)std::max<int64_t>(n, 1) * sizeof(T)));
+    void* q = (keep ? out : tmp).get((size_t)std::max<int64_t>(n, 1) * sizeof(T));
+    if (q) (keep ? outputs : scratch).push_back(q);
+    return static_cast<T*>(q);
   }
-  void drop(void* q) { tmp.drop(q); }
+  void drop(void* q) {
+    const auto it = std::find(scratch.begin(), scratch.end(), q);
+    if (it == scratch.end()) return;
+    scratch.erase(it);
+    tmp.drop(q);
+  }
   bool temp(size_t need) {
     if (need <= cub_bytes) return true;
-    if (cub) tmp.drop(cub);
-    cub = tmp.get(need);
+    drop(cub);
+    cub = get<char>((int64_t)need);
     cub_bytes = cub ? need : 0;
     return cub != nullptr;
   }
@@ -382,11 +397,11 @@ struct Mem {
     }                                                   \
   } while (0)
 
-int device_near_lists(Plan& p, const int2* d_near, int64_t npair, std::string& err) {
+int device_near_lists(Plan& p, const int2* d_near, int64_t npair, DeviceSlab& tmp, std::string& err) {
   const Tree &T = p.T, &S = p.S;
   Plan::NearOnDevice& o = p.nd;
   o = Plan::NearOnDevice();
-  Mem M;
+  Mem M(tmp, *p.dev_slab);
   const int64_t nc = T.ncell;
   auto up = [&](const std::vector<int32_t>& v, const int32_t** d) -> int {
     int32_t* q;
@@ -698,8 +713,7 @@ int device_near_lists(Plan& p, const int2* d_near, int64_t npair, std::string& e
   o.p2p_order = it.order;
   NL_CK(cudaDeviceSynchronize());
   o.on = true;
-  const std::vector<void*> kept = M.out.take();
-  p.dev_allocs.insert(p.dev_allocs.end(), kept.begin(), kept.end());
+  M.keep_outputs = true;
   return 0;
 }
 

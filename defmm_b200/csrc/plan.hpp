@@ -73,6 +73,8 @@ struct Slots {
   int64_t slot_of(int64_t c, int d) const;  // -1 when absent; d = -1 for LF
 };
 
+class DeviceSlab;
+
 struct Plan {
   // parameters
   int L = 0, P = 0, LL = 0, PP = 0, ncrit = 0, lvmax = -1;
@@ -177,9 +179,9 @@ struct Plan {
     const int32_t *red_first = nullptr, *red_n = nullptr;
     const int64_t *red_ptr = nullptr, *red_off = nullptr;
   } nd;
-  // the device allocations behind every dev_* array and nd above (pieces of
-  // them): the operator that owns the plan frees them
-  std::vector<void*> dev_allocs;
+  // where the device arrays dev_* and nd above are taken from: pieces that
+  // stay there, also when the build fails, until the owner releases it
+  DeviceSlab* dev_slab = nullptr;
   // sizes of the near-field lists wherever they were built
   int64_t near_chunks() const { return nd.on ? nd.nchunk : (int64_t)p2p_tfirst.size(); }
   int64_t near_items() const { return nd.on ? nd.p2p_items : (int64_t)p2p_order.size(); }

@@ -373,13 +373,7 @@ struct Arena {
 
 // Device arrays that stay with the plan, whatever comes of the walk.
 struct Keep {
-  Plan& p;
-  DeviceSlab slab;
-  explicit Keep(Plan& plan) : p(plan) {}
-  ~Keep() {
-    const std::vector<void*> v = slab.take();
-    p.dev_allocs.insert(p.dev_allocs.end(), v.begin(), v.end());
-  }
+  DeviceSlab& slab;
   template <typename T>
   T* get(size_t n) {
     return static_cast<T*>(slab.get(std::max<size_t>(1, n) * sizeof(T)));
@@ -433,7 +427,7 @@ int DeviceWalker::walk(Plan& p, LevelWalk& walk, std::string& err) {
   const Levels& v = p.lv;
   const int nlvl = v.nlvl;
   Arena A;
-  Keep K(p);
+  Keep K{*p.dev_slab};
   // cells per level (DFS order) and level-local indices, as the host walk
   std::vector<std::vector<int32_t>> lcT(nlvl), lcS(nlvl);
   std::vector<int32_t> locT(p.T.ncell), locS(p.S.ncell);
@@ -927,7 +921,7 @@ int DeviceWalker::walk(Plan& p, LevelWalk& walk, std::string& err) {
     }
     lv_near.clear();
     p.n_near = nn;
-    st = device_near_lists(p, all_near, nn, err);
+    st = device_near_lists(p, all_near, nn, A.slab, err);
     if (st == -5) {  // beyond device memory or 32-bit sort sizes: the host builds the lists
       std::vector<int2> near_h((size_t)nn);
       DW_CK(cudaMemcpy(near_h.data(), all_near, (size_t)nn * sizeof(int2), cudaMemcpyDeviceToHost));
@@ -1317,18 +1311,22 @@ __global__ void k_to_float(int64_t n, const double2* __restrict__ in, float2* __
     out[i] = make_float2(__double2float_rn(in[i].x), __double2float_rn(in[i].y));
 }
 
-int device_plan_tables(const Plan& p, double2* tables, double2* sig, double2* sig2, std::string& err) {
+int device_plan_tables(const Plan& p, double2* tables, double2* sig, double2* sig2, DeviceSlab& slab,
+                       std::string& err) {
   auto fail = [&](const char* what, cudaError_t e) {
     err = std::string("device tables: ") + what + ": " + cudaGetErrorString(e);
     cudaGetLastError();
     return -4;
   };
-  DeviceSlab tmp;
+  std::vector<void*> tmp;
   auto up = [&](const void* src, size_t bytes, void** dst) -> cudaError_t {
-    if (!(*dst = tmp.get(bytes))) return cudaErrorMemoryAllocation;
+    if (!(*dst = slab.get(bytes))) return cudaErrorMemoryAllocation;
+    tmp.push_back(*dst);
     return bytes ? cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
   };
-  auto release = [&]() { tmp.release(); };
+  auto release = [&]() {
+    for (void* q : tmp) slab.drop(q);
+  };
   cudaError_t e = cudaSuccess;
   const int64_t ntab = (int64_t)p.tab_fund.size();
   if (ntab) {

@@ -28,16 +28,19 @@ class DeviceSlab {
   DeviceSlab& operator=(const DeviceSlab&) = delete;
   ~DeviceSlab() { release(); }
 
-  // nullptr when out of device memory (the CUDA error is cleared)
-  void* get(size_t bytes) {
+  // nullptr when out of device memory (the CUDA error is cleared), or when no
+  // free piece serves and the slab is not to grow
+  void* get(size_t bytes, bool grow = true) {
     bytes = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
     if (bytes >= kBig) {
+      if (!grow) return nullptr;
       void* p = alloc(bytes);
       if (p) big_.push_back(p);
       return p;
     }
     for (auto it = free_.begin(); it != free_.end(); ++it)
       if (it->second >= bytes) return carve(it, bytes);
+    if (!grow) return nullptr;
     char* c = static_cast<char*>(alloc(std::max(bytes, grow_)));
     size_t size = std::max(bytes, grow_);
     if (!c) {

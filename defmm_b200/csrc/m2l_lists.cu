@@ -60,42 +60,55 @@ unsigned blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 int device_m2l_lists(const int64_t* ptr, int32_t* src, int64_t nent, int64_t nT, int64_t nS,
                      std::vector<int64_t>& atT, std::vector<int64_t>& atS, int64_t* cptr, int32_t* tlist,
                      int32_t* slist, DeviceSlab& slab, std::string& err) {
-  const int64_t nmax = std::max(nT, nS) + 1, na = (int64_t)std::max(atT.size(), atS.size());
+  const int64_t nmax = std::max(nT, nS) + 1, na = (int64_t)(atT.size() + atS.size());
   size_t scan = 0;
-  char* tmp = nullptr;
   cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, scan, (int32_t*)nullptr, (int32_t*)nullptr, nmax);
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t flag_b = up(nmax * 4), at_b = up(na * 8);
-  if (e == cudaSuccess && !(tmp = (char*)slab.get(2 * flag_b + 2 * at_b + scan))) e = cudaErrorMemoryAllocation;
+  const size_t flag_b = up(nmax * 4), at_b = up(na * 8), need = 2 * flag_b + 2 * at_b + scan;
+  DeviceSlab own;  // where the plan's slab has no room left: it would keep the scratch
+  char* tmp = (char*)slab.get(need, false);
+  char* const borrowed = tmp;
+  if (e == cudaSuccess && !tmp && !(tmp = (char*)own.get(need))) e = cudaErrorMemoryAllocation;
   int32_t *flag = (int32_t*)tmp, *rank = (int32_t*)(tmp + flag_b);
   int64_t *at = (int64_t*)(tmp + 2 * flag_b), *got = (int64_t*)(tmp + 2 * flag_b + at_b);
   void* cubtmp = tmp + 2 * flag_b + 2 * at_b;
-  auto ranks = [&](int64_t n, std::vector<int64_t>& v) -> cudaError_t {  // scan of flag[0, n], picked at v
+  std::vector<int64_t> both(atT);
+  both.insert(both.end(), atS.begin(), atS.end());
+  if (e == cudaSuccess && na) e = cudaMemcpy(at, both.data(), na * 8, cudaMemcpyHostToDevice);
+  auto ranks = [&](int64_t n, int64_t a0, int64_t a1) -> cudaError_t {  // scan of flag[0, n], picked at [a0, a1)
     size_t b = scan;
-    cudaError_t r = cub::DeviceScan::ExclusiveSum(cubtmp, b, flag, rank, n + 1);
-    if (r != cudaSuccess) return r;
-    if (v.empty()) return cudaSuccess;
-    if ((r = cudaMemcpy(at, v.data(), v.size() * 8, cudaMemcpyHostToDevice)) != cudaSuccess) return r;
-    k_pick<<<blocks((int64_t)v.size()), 256>>>((int64_t)v.size(), at, rank, got);
-    return cudaMemcpy(v.data(), got, v.size() * 8, cudaMemcpyDeviceToHost);
+    const cudaError_t r = cub::DeviceScan::ExclusiveSum(cubtmp, b, flag, rank, n + 1);
+    if (r == cudaSuccess && a1 > a0) k_pick<<<blocks(a1 - a0), 256>>>(a1 - a0, at + a0, rank, got + a0);
+    return r;
   };
   const unsigned ge = (unsigned)std::min<int64_t>(std::max<int64_t>(1, (nent + 255) / 256), 148 * 64);
   if (e == cudaSuccess) {
     k_flag_targets<<<blocks(nT + 1), 256>>>(ptr, nT, flag);
-    e = ranks(nT, atT);
-    k_compact_targets<<<blocks(nT + 1), 256>>>(ptr, nT, rank, cptr, tlist);
+    e = ranks(nT, 0, (int64_t)atT.size());
   }
-  if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, (nS + 1) * 4, 0);
+  if (e == cudaSuccess) {
+    k_compact_targets<<<blocks(nT + 1), 256>>>(ptr, nT, rank, cptr, tlist);
+    e = cudaMemsetAsync(flag, 0, (nS + 1) * 4, 0);
+  }
   if (e == cudaSuccess) {
     if (nent) k_flag_sources<<<ge, 256>>>(src, nent, flag);
-    e = ranks(nS, atS);
+    e = ranks(nS, (int64_t)atT.size(), na);
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) {  // the entries last: they are as they were when anything before fails
     if (nS) k_compact_sources<<<blocks(nS), 256>>>(nS, rank, slist);
     if (nent) k_rank_entries<<<ge, 256>>>(nent, rank, src);
+    e = cudaGetLastError();
   }
+  if (e == cudaSuccess && na) e = cudaMemcpy(both.data(), got, na * 8, cudaMemcpyDeviceToHost);
   const cudaError_t d = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = d;
-  if (tmp) slab.drop(tmp);
-  if (e == cudaSuccess) return 0;
+  if (borrowed) slab.drop(borrowed);
+  if (e == cudaSuccess) {
+    std::copy(both.begin(), both.begin() + atT.size(), atT.begin());
+    std::copy(both.begin() + atT.size(), both.end(), atS.begin());
+    return 0;
+  }
   cudaGetLastError();
   err = std::string("M2L list compaction: ") + cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? -5 : -4;

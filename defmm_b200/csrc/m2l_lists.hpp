@@ -14,8 +14,8 @@ namespace dfb {
 // into src, in cptr with one past the last), the source slots that occur in
 // slist, both in slot order, and src rewritten to positions in slist.
 // atT / atS: slot numbers (<= nT / <= nS), replaced by how many listed slots
-// lie before each.  Room: nT + 1, nT and nS entries; scratch from slab.  0, -4
-// or -5 (out of device memory) with err set.
+// lie before each.  Room: nT + 1, nT and nS entries; scratch is what slab has
+// free, or given back.  0, -4 or -5 (out of device memory) with err set.
 int device_m2l_lists(const int64_t* ptr, int32_t* src, int64_t nent, int64_t nT, int64_t nS,
                      std::vector<int64_t>& atT, std::vector<int64_t>& atS, int64_t* cptr, int32_t* tlist,
                      int32_t* slist, DeviceSlab& slab, std::string& err);

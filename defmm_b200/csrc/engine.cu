@@ -895,12 +895,18 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
         int c1 = c0 + 1;
         while (c1 < nc && cS[c1 + 1] - cS[c0] <= h->f_cap) c1++;
         const int64_t fs0 = cS[c0], fs1 = cS[c1], ts0 = cT[c0], ts1 = cT[c1];
+        // slices of one size (the last ones may be short or empty): the list
+        // entries before each in one strided copy, those before the end known
         constexpr int kSlices = 16;
-        int64_t ent[kSlices + 1] = {0};  // list entries before each slice
-        for (int i = 0; i <= kSlices && ts1 > ts0 && fs1 > fs0; i++)
-          CK(cudaMemcpy(&ent[i], d.m2l_cptr + ts0 + (ts1 - ts0) * i / kSlices, 8, cudaMemcpyDeviceToHost));
+        const int64_t step = (ts1 - ts0 + kSlices - 1) / kSlices;
+        int64_t ent[kSlices + 1];
+        if (ts1 > ts0 && fs1 > fs0) {
+          std::fill(ent, ent + kSlices + 1, p.m2l_ptr[p.sT.cone_begin[l][c1]]);
+          CK(cudaMemcpy2D(ent, 8, d.m2l_cptr + ts0, step * 8, 8, (ts1 - ts0 + step - 1) / step,
+                          cudaMemcpyDeviceToHost));
+        }
         for (int i = 0; i < kSlices && ts1 > ts0 && fs1 > fs0; i++) {
-          const int64_t a0 = ts0 + (ts1 - ts0) * i / kSlices, a1 = ts0 + (ts1 - ts0) * (i + 1) / kSlices;
+          const int64_t a0 = ts0 + step * i, a1 = std::min(ts1, a0 + step);
           if (a1 <= a0) continue;
           const int c = i % 4;
           rec(h, 2 * PH_M2L);

@@ -91,7 +91,7 @@ struct defmm_handle {
   const int32_t* d_p2p_order = nullptr;
   const int32_t *d_p2p_item_chunk = nullptr, *d_sym_item_chunk = nullptr;
   const int64_t *d_p2p_chunk_items = nullptr, *d_sym_chunk_items = nullptr;
-  double2* d_tpart = nullptr;  // near-field item partial sums (32 per item and part)
+  DevBuf tpart;  // near-field item partial sums (32 per item and part), resident layout
   int p2p_split = 1, sym_split = 1;  // parts per near-field item (near_split)
   unsigned long long* d_queue = nullptr;
   // symmetric near field (Plan::self_*, sym_*, red_*)
@@ -256,6 +256,7 @@ void free_plan_device(defmm_handle* h) {
   free_buf(h->rout);
   free_buf(h->chk);
   free_buf(h->pscr);
+  free_buf(h->tpart);
   free_grouped(h);
   h->layout = 0;
   h->use_sym = false;
@@ -463,13 +464,6 @@ int upload_plan(defmm_handle* h) {
     const int64_t pairs = p.i_near;
     h->p2p_split = near_split(h->nsm, p.near_items(), p.near_chunks(), pairs, (int64_t)p.T.perm.size());
     h->sym_split = near_split(h->nsm, p.near_sym_items(), p.near_chunks(), pairs / 2, (int64_t)p.T.perm.size());
-    const size_t nitem = (size_t)std::max<int64_t>(
-        1, std::max(p.near_items() * h->p2p_split, p.near_sym_items() * h->sym_split));
-    void* tp = nullptr;
-    CK(cudaMalloc(&tp, nitem * 32 * sizeof(double2)));
-    h->plan_allocs.push_back(tp);
-    h->dev_bytes += nitem * 32 * sizeof(double2);
-    h->d_tpart = static_cast<double2*>(tp);
     void* qc = nullptr;
     CK(cudaMalloc(&qc, 2 * sizeof(unsigned long long)));  // P2P (stream 2), M2L (main stream)
     h->plan_allocs.push_back(qc);
@@ -533,6 +527,7 @@ int prepare_tables(defmm_handle* h) {
   free_buf(h->sig2);
   free_buf(h->ptab);
   free_buf(h->pscr);
+  free_buf(h->tpart);
   free_grouped(h);
   h->layout = 0;
   h->use_sym = false;
@@ -639,12 +634,22 @@ int64_t largest_cone(const Plan& p) {
   return need;
 }
 
-// Device bytes of the resident layout: every slot's M and L, charges, the
-// smallest F batch.
+// Parts of a near-field item that one right-hand side runs (the mixed path's
+// FP32 sums run over whole items), and the bytes of their partial sums.
+int p2p_parts(const defmm_handle* h, int split) { return h->precision == DEFMM_PRECISION_FP64 ? split : 1; }
+size_t tpart_bytes(const defmm_handle* h) {
+  const int64_t n = std::max(h->plan.near_items() * p2p_parts(h, h->p2p_split),
+                             h->plan.near_sym_items() * p2p_parts(h, h->sym_split));
+  return (size_t)std::max<int64_t>(1, n) * 32 * sizeof(double2);
+}
+
+// Device bytes of the resident layout: every slot's M and L, charges, near-field
+// partial sums, the smallest F batch.
 size_t resident_bytes(const defmm_handle* h) {
   const Plan& p = h->plan;
   const size_t cs = h->precision == DEFMM_PRECISION_FP64 ? 16 : 8;
-  return (size_t)(p.sS.n + p.sT.n) * p.LL * cs + p.S.perm.size() * cs + (size_t)largest_cone(p) * p.PP * cs;
+  return (size_t)(p.sS.n + p.sT.n) * p.LL * cs + p.S.perm.size() * cs + tpart_bytes(h) +
+         (size_t)largest_cone(p) * p.PP * cs;
 }
 
 // Resident layout: M and L of every slot.  Releases a grouped layout first.
@@ -659,7 +664,8 @@ int prepare_resident(defmm_handle* h) {
   int st;
   const int64_t nS = (int64_t)p.S.perm.size();
   if ((st = ensure(h, h->M, std::max<int64_t>(1, p.sS.n) * p.LL * cs)) ||
-      (st = ensure(h, h->Lx, std::max<int64_t>(1, p.sT.n) * p.LL * cs)) || (st = ensure(h, h->q, nS * cs)))
+      (st = ensure(h, h->Lx, std::max<int64_t>(1, p.sT.n) * p.LL * cs)) || (st = ensure(h, h->q, nS * cs)) ||
+      (st = ensure(h, h->tpart, tpart_bytes(h))))
     return st;
   // symmetric near field when its scratch takes at most 70% of the free
   // memory and can be allocated (otherwise every interaction is evaluated
@@ -730,6 +736,7 @@ int prepare_grouped(defmm_handle* h, int R) {
   free_buf(h->F);
   free_buf(h->q);
   free_buf(h->pscr);
+  free_buf(h->tpart);
   h->use_sym = false;
   free_grouped(h);
   h->layout = 0;
@@ -857,26 +864,25 @@ int run_gemv(defmm_handle* h, const double2* qin, double2* out, cudaStream_t s) 
   CK(cudaEventRecord(ready, s));
   CK(cudaStreamWaitEvent(sn, ready, 0));
   if (h->events) cudaEventRecord(h->ev[2 * PH_P2P], sn);
-  // the mixed path's FP32 sums run over whole items
-  const int p2p_split = fp64 ? h->p2p_split : 1, sym_split = fp64 ? h->sym_split : 1;
+  const int p2p_split = p2p_parts(h, h->p2p_split), sym_split = p2p_parts(h, h->sym_split);
   if (h->use_sym) {  // own leaves, then symmetric blocks, then the mirrored partial sums
     dfb::launch_p2p(fp64, d, p.near_self_items(), h->d_self_order, nullptr, h->d_tfirst, h->d_tn,
                     h->d_self_ptr, h->d_self_sfirst, h->d_self_sn, h->q.p, (double2*)h->pnear.p, nullptr,
                     1, h->d_queue, h->nsm, sn);
     dfb::launch_p2p_sym(fp64, d, p.near_sym_items(), h->d_sym_order, h->d_sym_item_chunk, h->d_tfirst,
-                        h->d_tn, h->d_sym_ptr, h->d_sym_sfirst, h->d_sym_sn, h->d_sym_soff, h->q.p, h->d_tpart,
-                        h->pscr.p, sym_split, h->d_queue, h->nsm, h->p2p_bps[fp64 ? 0 : 1], sn);
-    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_sym_chunk_items, h->d_tpart, sym_split,
-                          (double2*)h->pnear.p, h->nsm, sn);
+                        h->d_tn, h->d_sym_ptr, h->d_sym_sfirst, h->d_sym_sn, h->d_sym_soff, h->q.p,
+                        (double2*)h->tpart.p, h->pscr.p, sym_split, h->d_queue, h->nsm, h->p2p_bps[fp64 ? 0 : 1], sn);
+    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_sym_chunk_items, (const double2*)h->tpart.p,
+                          sym_split, (double2*)h->pnear.p, h->nsm, sn);
     dfb::launch_p2p_reduce(fp64, p.near_red_leaves(), h->d_red_first, h->d_red_n, h->d_red_ptr,
                            h->d_red_off, h->pscr.p, (double2*)h->pnear.p, h->nsm, sn);
     nl_ += (p.near_self_items() ? 1 : 0) + (p.near_sym_items() ? 2 : 0) + (p.near_red_leaves() ? 1 : 0);
   } else {  // every interaction from the target side, in items
     dfb::launch_p2p(fp64, d, p.near_items(), h->d_p2p_order, h->d_p2p_item_chunk, h->d_tfirst, h->d_tn,
-                    h->d_p2p_ptr, h->d_sfirst, h->d_sn, h->q.p, (double2*)h->pnear.p, h->d_tpart, p2p_split,
-                    h->d_queue, h->nsm, sn);
-    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, h->d_tpart, p2p_split,
-                          (double2*)h->pnear.p, h->nsm, sn);
+                    h->d_p2p_ptr, h->d_sfirst, h->d_sn, h->q.p, (double2*)h->pnear.p, (double2*)h->tpart.p,
+                    p2p_split, h->d_queue, h->nsm, sn);
+    dfb::launch_p2p_items(h->nchunk, h->d_tfirst, h->d_tn, h->d_p2p_chunk_items, (const double2*)h->tpart.p,
+                          p2p_split, (double2*)h->pnear.p, h->nsm, sn);
     nl_ += p.near_items() ? 2 : 0;
   }
   if (h->events) cudaEventRecord(h->ev[2 * PH_P2P + 1], sn);
@@ -1287,7 +1293,7 @@ int run_gemv_grouped(defmm_handle* h, const double2* qin, int64_t stride_in, dou
 // Device bytes held by the expansion layout of the current precision.
 size_t layout_bytes(const defmm_handle* h) {
   const GroupedLayout& g = h->gl;
-  size_t b = h->M.bytes + h->Lx.bytes + h->F.bytes + h->q.bytes + h->pscr.bytes;
+  size_t b = h->M.bytes + h->Lx.bytes + h->F.bytes + h->q.bytes + h->pscr.bytes + h->tpart.bytes;
   for (const DevBuf* x : {&g.Mg, &g.Lg, &g.Mlf, &g.Llf, &g.F, &g.q, &g.pnear, &g.pfar, &g.tpart}) b += x->bytes;
   return b;
 }

@@ -624,14 +624,26 @@ int prepare_tables(defmm_handle* h) {
   return 0;
 }
 
-// Largest cone (source slots) of any precomputed level: the smallest F batch.
-int64_t largest_cone(const Plan& p) {
+// Source slots per level and cone that F batches hold: those in some M2L list
+// (before the upload has listed them: all).
+const std::vector<int64_t>& f_slots(const defmm_handle* h, int l) {
+  return h->uploaded ? h->sU[l] : h->plan.sS.cone_begin[l];
+}
+
+// Largest cone of any precomputed level (the smallest F batch) and largest
+// level (the largest one worth having).
+int64_t largest_cone(const defmm_handle* h) {
   int64_t need = 1;
-  for (int l = 0; l < p.lv.nlvl; l++) {
-    const auto& cS = p.sS.cone_begin[l];
+  for (int l = 0; l < h->plan.lv.nlvl; l++) {
+    const auto& cS = f_slots(h, l);
     for (size_t c = 0; c + 1 < cS.size(); c++) need = std::max(need, cS[c + 1] - cS[c]);
   }
   return need;
+}
+int64_t largest_level(const defmm_handle* h) {
+  int64_t want = 0;
+  for (int l = 0; l < h->plan.lv.nlvl; l++) want = std::max(want, f_slots(h, l).back() - f_slots(h, l).front());
+  return want;
 }
 
 // Parts of a near-field item that one right-hand side runs (the mixed path's
@@ -649,7 +661,7 @@ size_t resident_bytes(const defmm_handle* h) {
   const Plan& p = h->plan;
   const size_t cs = h->precision == DEFMM_PRECISION_FP64 ? 16 : 8;
   return (size_t)(p.sS.n + p.sT.n) * p.LL * cs + p.S.perm.size() * cs + tpart_bytes(h) +
-         (size_t)largest_cone(p) * p.PP * cs;
+         (size_t)largest_cone(h) * p.PP * cs;
 }
 
 // Resident layout: M and L of every slot.  Releases a grouped layout first.
@@ -689,11 +701,7 @@ int prepare_resident(defmm_handle* h) {
   }
   // F batch buffer: at least the largest cone of any level, at most about
   // half of the free memory
-  int64_t need = largest_cone(p), want = 0;
-  for (int l = 0; l < p.lv.nlvl; l++) {
-    const auto& cS = p.sS.cone_begin[l];
-    want = std::max(want, cS.back() - cS.front());
-  }
+  const int64_t need = largest_cone(h), want = largest_level(h);
   size_t fr = 0, tot = 0;
   CK(cudaMemGetInfo(&fr, &tot));
   const size_t per = (size_t)p.PP * cs;
@@ -774,10 +782,8 @@ int prepare_grouped(defmm_handle* h, int R) {
   // F batch: at least the largest cone, at most a quarter of the free memory
   // (and 32 GB)
   const size_t fper = (size_t)R * p.PP * cs;
-  const int64_t need = largest_cone(p);
+  const int64_t need = largest_cone(h), want = largest_level(h);
   int64_t cap = (int64_t)(std::min<size_t>(fr / 4, (size_t)32 << 30) / fper);
-  int64_t want = 0;
-  for (int l = 0; l < v.nlvl; l++) want = std::max(want, p.sS.cone_begin[l].back() - p.sS.cone_begin[l].front());
   cap = std::min(cap, std::max(want, need));
   if (cap < need) return h->fail(DEFMM_ERR_MEMORY, "not enough device memory for one cone of spectra");
   g.f_cap = cap;

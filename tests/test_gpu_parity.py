@@ -587,3 +587,26 @@ def test_blocks_at_high_orders(order, gpu):
             A.set_blocking(R, 1)
             P = A.matvec(Q[:R])
             assert np.array_equal(P[1], one)
+
+
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_f_buffer_holds_listed_slots_only(nrhs, gpu):
+    # a third of the source slots are in no M2L list: of the device memory that
+    # a matvec takes beyond the upload's, what is left after expansions,
+    # vectors and spectra has room for the F of a level's listed slots, not all
+    src, trg = W.gaussian_blobs(15001, seed=1).points, W.sphere_surface(7999, seed=2).points * 0.45
+    A = make(src, trg, 4, 40, 2 * np.pi * 6 / np.sqrt(3))
+    A.set_blocking(nrhs, 1 if nrhs > 1 else 0)
+    cells = A.tree("S")[0]
+    per_level = np.bincount(cells[:, 3], weights=cells[:, 7]).astype(int)  # slots, level-major
+    assert per_level.sum() == A.info("slots_S")
+    ends = np.concatenate([[0], np.cumsum(per_level)])
+    listed = np.histogram(np.unique(A.m2l_entries()[1]), ends)[0].max()
+    A.upload()
+    before = A.info("device_bytes")
+    q = W.charges(len(src), 1)
+    A.matvec(q if nrhs == 1 else np.stack([q] * nrhs))
+    i = A.info()
+    known = 16 * (nrhs * ((i["slots_S"] + i["slots_T"]) * 64 + 3 * len(src) + 3 * len(trg)) + i["permuted_spectra"] * 343)
+    rest = 16 * 343 * nrhs * listed + nrhs * (4 << 20)  # signatures and near-field partial sums: some MB
+    assert i["device_bytes"] - before <= known + rest < known + 0.9 * 16 * 343 * nrhs * per_level.max()

@@ -110,9 +110,11 @@ __global__ void k_scatter(const double2* __restrict__ pnear, const double2* __re
 // tile (expansion entries lane + 32 e, all S slots, so signatures and results
 // are read and written at unit stride) over the chunk's points: per point R
 // loads of Z and S broadcast loads of W feed 2 R S FMAs.  Latency bounds it
-// (the signatures' loads), so an FP64 chunk is small enough for 4 CTAs per SM:
-// sphere 250k FP64 5.7 -> 4.0 ms against entries R lane .. R lane + R - 1 and
-// chunks of 64 points.  FP32 chunks hold 64 points where they fit: their sums
+// (the signatures' loads), so an FP64 chunk's Z takes at most 40 KB: with the
+// offsets, the basis and W 3 CTAs fit an SM at orders 4 and 5 (57,856 and 57,600
+// bytes; 76,288 with several right-hand sides at order 4), 4 at order 6, 5 above.
+// Sphere 250k FP64 5.7 -> 4.0 ms against entries R lane .. R lane + R - 1 and
+// chunks of 64 points (2 CTAs).  FP32 chunks hold 64 points where they fit: their sums
 // are rounded chunk by chunk, and results keep their bits (spheroid 500k mixed
 // order 6 9.1 -> 7.0 ms, 5.5 with chunks of 40).
 template <typename T, int L>
@@ -131,6 +133,9 @@ struct P2MCfg {
     return sizeof(T) * (size_t)NPB * LLP + sizeof(double) * NPB * 3 + sizeof(T) * NPB * 3 * L +
            sizeof(C) * 4 * NPB * S * (R > 1 ? 2 : 1) + sizeof(C) * (size_t)NPB * R;
   }
+  // W follows Z, the offsets and the basis: an odd chunk could misalign it
+  static_assert((sizeof(T) * NPB * LLP + sizeof(double) * NPB * 3 + sizeof(T) * NPB * 3 * L) % sizeof(C) == 0,
+                "W blocks are read as complex values");
 };
 
 template <typename T, int L, int SS>
@@ -1990,7 +1995,7 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float x) {
 }
 
 // Mixed-precision interaction with FP32 compensated accumulators (the FP64
-// path keeps p2p_pair<false>).  1/r: approximate FP64 reciprocal square root
+// path: green64_r).  1/r: approximate FP64 reciprocal square root
 // refined once in FP64 (relative error ~1e-14), used for k r, and rounded to
 // FP32 for 1/(4 pi r).  k r = n pi + x with n read from the
 // low mantissa bits of k r / pi + 1.5 * 2^52 (exact for k r / pi < 2^51) and
@@ -3053,7 +3058,7 @@ struct Launch {
   static void p2m(const DevPlan& dp, const int32_t* leaves, int n, const void* q, const void* sig2, void* M, int R,
                   int d0, int d1, cudaStream_t s) {
     if (!n) return;
-    // parts until there are 16 CTAs per SM (4 are resident): the three P2M
+    // parts until there are 16 CTAs per SM (3 to 6 are resident): the three P2M
     // launches (95, 364 and 938 leaves) of blobs of 15,001 points, order 4,
     // three right-hand sides, FP64 took 134 us whole and take 95 us in parts
     const int split = std::max(1, std::min(4, 148 * 16 / n));
